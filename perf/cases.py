@@ -244,3 +244,83 @@ def run(s):
     o = ops.fmha_fwd_splitkv(s["q"], s["k"], s["v"], seqlen_k=s["seqlen"], block_table=s["table"], cu_seqlens_q=s["cu_q"],
                              max_seqlen_q=s["max_q"], causal=True)
     return {"o": o, "q": s["q"], "k_cache": s["k"], "v_cache": s["v"]}
+
+
+# ---- the same in 64 bits ----------------------------------------------------------------------------------------------
+def _rope64(x, cos, sin):
+    """Interleaved pairs of x [n, heads, d] rotated by the n rows of cos / sin."""
+    x, c, s = x.double(), cos.double()[:, None], sin.double()[:, None]
+    a, b = x[..., 0::2], x[..., 1::2]
+    return torch.stack((a * c - b * s, a * s + b * c), -1).flatten(-2)
+
+
+def _attend64(case, q, k, v, bias=None, slopes=None, scale=None):
+    """Attention of one sequence, q [nq, hq, d] over k, v [nk, hkv, d]: (o, lse [hq, nq]), a block of rows of one head at a time."""
+    (nq, hq, d), nk, group = q.shape, k.shape[0], q.shape[1] // k.shape[1]
+    o = torch.empty((nq, hq, d), dtype=torch.float64, device=q.device)
+    lse = torch.empty((hq, nq), dtype=torch.float64, device=q.device)
+    step, keys = max(1, (1 << 27) // nk), torch.arange(nk, device=q.device)
+    for h in range(hq):
+        if h % group == 0:
+            kh, vh = k[:, h // group].double(), v[:, h // group].double()
+        for r in range(0, nq, step):
+            rows = torch.arange(r, min(nq, r + step), device=q.device)[:, None] + (nk - nq)
+            x = (q[r:r + step, h].double() @ kh.T) * (scale or d ** -0.5)
+            if case.get("cap", 0.0) > 0:
+                x = case["cap"] * torch.tanh(x / case["cap"])
+            if bias is not None:
+                x += bias[0, h if bias.shape[1] > 1 else 0, r:r + step].double()
+            if slopes is not None:
+                x -= slopes[0, h].double() * (rows - keys).abs()
+            if case.get("mask", "causal" if nq > 1 else "none") != "none":
+                x.masked_fill_(keys > rows, float("-inf"))
+                if case.get("mask") == "window":
+                    x.masked_fill_(keys < rows - case["window"], float("-inf"))
+            lse[h, r:r + step] = torch.logsumexp(x, -1)
+            o[r:r + step, h] = torch.softmax(x, -1) @ vh
+    return o, lse
+
+
+def exact(case, seed):
+    nq, nk = _lens(case)
+    if case["hq"] * sum(q * k for q, k in zip(nq, nk)) > 2.5e10:
+        return None
+    s = prepare(case, seed)
+    op = case["op"]
+    if op == "dense":
+        kw = s["kw"]
+        parts = [_attend64(case, s["q"][i], s["k"][i], s["v"][i], kw.get("bias"), kw.get("alibi_slopes")) for i in range(case["batch"])]
+        o, lse = torch.stack([p[0] for p in parts]), torch.stack([p[1] for p in parts])
+        return (o, lse) if case["lse"] else o
+    cq = [sum(nq[:i]) for i in range(len(nq) + 1)]
+    if op == "varlen":
+        sc = s.get("scales")
+        parts = [_attend64(case, s["q"][a:b], s["k"][a:b], s["v"][a:b], scale=sc and sc["scale_s"]) for a, b in zip(cq, cq[1:])]
+        o, lse = torch.cat([p[0] for p in parts]), torch.cat([p[1] for p in parts], 1)
+        if sc:
+            o *= sc["scale_p"] * sc["scale_o"]
+        return (o, lse) if case["lse"] else o
+
+    def cached(pool, b):
+        if not case["page"]:
+            return pool[b, :nk[b]]
+        return pool[s["table"][b, :-(-nk[b] // case["page"])].long()].flatten(0, 1)[:nk[b]]
+
+    q, out = s["q"].flatten(0, 1) if op == "decode" else s["q"], {}
+    if op == "append":
+        pos = torch.cat([torch.arange(k - n, k) for n, k in zip(nq, nk)]).to(q.device)
+        knew = _rope64(s["knew"], s["cos"][pos], s["sin"][pos])
+        q = _rope64(q, s["cos"][pos], s["sin"][pos])
+        out = {"q": q, "k_cache": None, "v_cache": None}  # (whole pools: copies of the new rows, and the rest as it was)
+    parts = []
+    for b in range(case["batch"]):
+        k, v = cached(s["k"], b).double(), cached(s["v"], b).double()
+        if op == "append":
+            k[nk[b] - nq[b]:], v[nk[b] - nq[b]:] = knew[cq[b]:cq[b + 1]], s["vnew"][cq[b]:cq[b + 1]].double()
+        parts.append(_attend64(case, q[cq[b]:cq[b + 1]] if op != "decode" else s["q"][b], k, v))
+    o, lse = torch.cat([p[0] for p in parts]), torch.cat([p[1] for p in parts], 1)
+    if op == "append":
+        return {"o": o, **out}
+    if op == "decode":
+        return o.view(s["q"].shape)
+    return (o, lse) if case["lse"] else o
