@@ -3,7 +3,8 @@
 // (attention_kernels/fmha_fwd_split_kv_combine/fmha_fwd_split_kv_combine_jinja.h:125-140): lse_acc
 // [bs,hq,S,rows], o_acc [bs,hq,S,rows,dv].  The strided form also reads partials gathered from several GPUs
 // ([rank][...] layouts) and can leave the result in fp32, which is what a rank contributes to such a gather.
-// One warp per (batch, head, row); HBM-bound on o_acc (read once) -- a few MB, so launch latency dominates.
+// o_acc is read once and is a few MB at most, so what bounds the kernel is its chain of memory round trips: one warp per
+// (batch, head, row) when a row has few splits, several warps per row otherwise (see combine_wide_kernel).
 #include "kernels.h"
 
 namespace fck {
@@ -120,6 +121,121 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineDev p) {
     if (p.lse && lane == 0) p.lse[item] = m + logf(sum);
 }
 
+// Several warps per row (one CTA = one row), for rows with many splits: a warp that walks 94 splits four rows at a time
+// pays a memory round trip for every four.  Warp w takes splits w, w + W, ...; it requests its first kAhead rows before
+// it has seen any LSE (a split without keys may hold anything: its row is dropped by its weight of zero, not multiplied),
+// so that a row of W * kAhead splits costs two round trips -- LSE and partials together, then nothing but shared memory.
+// Merging one token of 32 heads over 128 split slots, 94 in use: 16.4 us with one warp per row, 3.3 us with 16 (back to
+// back in a graph; 24.5 us alone behind its split kernel before).
+template <typename T, int W>
+__global__ void __launch_bounds__(W * 32) combine_wide_kernel(const CombineDev p) {
+    constexpr int kAhead = 4;
+    extern __shared__ float4 part[];  // [W][dv / 4]: the warps' weighted sums
+    pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t item = blockIdx.x;
+    const int r = (int)(item % p.rows);
+    const int64_t bh = item / p.rows;
+    const int h = (int)(bh % p.hq);
+    const int64_t b = bh / p.hq;
+    const int S = p.S;
+    const float* lrow = p.lse_acc + b * p.lb + h * p.lh + r * p.lr;
+    const float* obase = p.o_acc + b * p.ob + h * p.oh + r * p.orr;
+    const int nvec = p.dv >> 2;
+    const bool c0 = lane < nvec, c1 = lane + 32 < nvec;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float ninf = -INFINITY;
+
+    float4 x[kAhead][2];
+    auto fetch = [&](int j0) {  // this warp's splits j0 .. j0 + kAhead - 1
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int s = (j0 + u) * W + warp;
+            const float4* src = reinterpret_cast<const float4*>(obase + (int64_t)s * p.os);
+            x[u][0] = (s < S && c0) ? src[lane] : zero;
+            x[u][1] = (s < S && c1) ? src[lane + 32] : zero;
+        }
+    };
+    fetch(0);
+    float mine = lane * W + warp < S ? lrow[(int64_t)(lane * W + warp) * p.ls] : ninf;  // lane j: split j * W + warp
+    // maximum and sum of weights over all splits (every warp for itself: they are at most a few loads per lane)
+    float l4[4], m = ninf;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        l4[u] = lane + 32 * u < S ? lrow[(int64_t)(lane + 32 * u) * p.ls] : ninf;
+        m = fmaxf(m, l4[u]);
+    }
+    for (int s = lane + 128; s < S; s += 32) m = fmaxf(m, lrow[s * p.ls]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    T* orow = (T*)p.o + ((b * p.rows + r) * p.hq + h) * (int64_t)p.dv;
+    if (m == ninf) {  // no split saw a key: O = 0, LSE = -inf (the same in every warp)
+        for (int c = threadIdx.x; c < nvec; c += W * 32) Out4<T>::store(orow + 4 * c, zero);
+        if (p.lse && threadIdx.x == 0) p.lse[item] = ninf;
+        return;
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) sum += (l4[u] == ninf) ? 0.f : expf(l4[u] - m);
+    for (int s = lane + 128; s < S; s += 32) {
+        const float ls = lrow[s * p.ls];
+        sum += (ls == ninf) ? 0.f : expf(ls - m);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    const float inv = 1.f / sum;
+
+    float4 acc[2] = {zero, zero};
+    for (int j0 = 0; j0 * W + warp < S; j0 += kAhead) {
+        if (j0 > 0) {
+            if ((j0 & 31) == 0) mine = (j0 + lane) * W + warp < S ? lrow[(int64_t)((j0 + lane) * W + warp) * p.ls] : ninf;
+            fetch(j0);
+        }
+        const float wl = (mine == ninf) ? 0.f : expf(mine - m) * inv;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const float w = __shfl_sync(0xffffffffu, wl, (j0 + u) & 31);
+            if (w == 0.f) continue;  // (warp-uniform)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                acc[j].x += w * x[u][j].x;
+                acc[j].y += w * x[u][j].y;
+                acc[j].z += w * x[u][j].z;
+                acc[j].w += w * x[u][j].w;
+            }
+        }
+    }
+    if (c0) part[warp * nvec + lane] = acc[0];
+    if (c1) part[warp * nvec + lane + 32] = acc[1];
+    __syncthreads();
+    for (int c = threadIdx.x; c < nvec; c += W * 32) {
+        float4 t = part[c];
+#pragma unroll
+        for (int w = 1; w < W; ++w) {
+            const float4 y = part[w * nvec + c];
+            t.x += y.x; t.y += y.y; t.z += y.z; t.w += y.w;
+        }
+        Out4<T>::store(orow + 4 * c, t);
+    }
+    if (p.lse && threadIdx.x == 0) p.lse[item] = m + logf(sum);
+}
+
+template <typename T>
+cudaError_t launch_t(const CombineDev& d, cudaStream_t stream) {
+    // Warps per row: as many as still find two splits each, while the rows together stay within 16 warps per SM; more
+    // warps than that only queue, and the other rows hide a row's round trips.  Measured (us with 1 / 4 / 8 / 16 warps,
+    // dv 128): 32 rows x 128 slots 16.4 / 4.9 / 3.7 / 3.3; 256 x 75 9.6 / 4.1 / 3.7 / 4.4; 512 x 20 4.2 / 3.1 / 3.6 /
+    // 6.0; 2048 x 16 4.4 / 5.5 / 9.5 / 18; 2048 x 6 3.6 / 5.4 / 9.1 / 17.
+    const int64_t warps_ok = (int64_t)sm_count() * 16 / (d.items > 0 ? d.items : 1);
+    const dim3 g((unsigned)d.items);
+    const size_t row = d.dv * sizeof(float);
+    if (warps_ok >= 16 && d.S > 32) return launch_dependent(combine_wide_kernel<T, 16>, g, dim3(512), 16 * row, stream, d);
+    if (warps_ok >= 8 && d.S > 16) return launch_dependent(combine_wide_kernel<T, 8>, g, dim3(256), 8 * row, stream, d);
+    if (warps_ok >= 4 && d.S > 8) return launch_dependent(combine_wide_kernel<T, 4>, g, dim3(128), 4 * row, stream, d);
+    const int warps = 4;
+    return launch_dependent(combine_kernel<T>, dim3((unsigned)((d.items + warps - 1) / warps)), dim3(warps * 32), 0, stream, d);
+}
+
 }  // namespace
 
 int launch_combine(const CombineParams& p, cudaStream_t stream) {
@@ -142,12 +258,9 @@ int launch_combine(const CombineParams& p, cudaStream_t stream) {
         d.orr = p.dv; d.os = p.rows * p.dv; d.oh = p.num_splits * d.os; d.ob = p.hq * d.oh;
     }
     if (d.items == 0) return FLASHCK_OK;
-    const int warps = 4;
-    const unsigned grid = (unsigned)((d.items + warps - 1) / warps);
-    const dim3 g(grid), b(warps * 32);
-    if (p.dtype == FLASHCK_DTYPE_BFLOAT16) FCK_CUDA(launch_dependent(combine_kernel<__nv_bfloat16>, g, b, 0, stream, d));
-    else if (p.dtype == FLASHCK_DTYPE_FLOAT16) FCK_CUDA(launch_dependent(combine_kernel<__half>, g, b, 0, stream, d));
-    else FCK_CUDA(launch_dependent(combine_kernel<float>, g, b, 0, stream, d));
+    if (p.dtype == FLASHCK_DTYPE_BFLOAT16) FCK_CUDA(launch_t<__nv_bfloat16>(d, stream));
+    else if (p.dtype == FLASHCK_DTYPE_FLOAT16) FCK_CUDA(launch_t<__half>(d, stream));
+    else FCK_CUDA(launch_t<float>(d, stream));
     return FLASHCK_OK;
 }
 

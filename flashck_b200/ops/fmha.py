@@ -452,9 +452,8 @@ def fmha_fwd_splitkv_combine(lse_acc: torch.Tensor, o_acc: torch.Tensor, dtype: 
             rc = _lib.lib().FmhaFwdSplitKVCombineStrided(_ptr(lse_acc), _ptr(o_acc), _ptr(o), _ptr(lse), bs, rows, hq, dv,
                                                          S, ls, os_, code, _stream())
         else:
-            # group mode is signalled by a non-null seqstart pointer; its contents are not needed by the combine
-            marker = torch.zeros(1, dtype=torch.int64, device=o_acc.device) if varlen else None
-            rc = _lib.lib().FmhaFwdSplitKVCombine(_ptr(lse_acc), _ptr(o_acc), _ptr(o), _ptr(marker), bs, rows, hq, dv,
+            # (no seqstart pointer in either mode: group mode only means one batch row, which varlen workspaces have)
+            rc = _lib.lib().FmhaFwdSplitKVCombine(_ptr(lse_acc), _ptr(o_acc), _ptr(o), None, bs, rows, hq, dv,
                                                   rows, S, _stream(), _ptr(lse), code)
     _lib.check(rc, "FmhaFwdSplitKVCombine")
     if varlen and out is None:
