@@ -7,8 +7,8 @@
 // rows per kv head (the "split modes" described at Sm100Dev and at the kernel template).
 //
 // Persistent kernel: one CTA per SM (384 threads; it owns all 512 TMEM columns) walks a work list that every CTA
-// derives on chip from the sequence lengths: items sorted by decreasing row-block index (decreasing cost under a
-// causal mask), dealt to the CTAs in snake order.  A work item is two 128-row Q tiles that share their K/V tiles:
+// derives on chip from the sequence lengths: items sorted by decreasing cost and dealt by the CTAs' loads (long lists: in
+// snake order; more than kMaxGroups row blocks: by decreasing row-block index).  A work item is two 128-row Q tiles that share their K/V tiles:
 // the same rows of two neighbouring q heads of a GQA group when the group size is even (both tiles then run the
 // same number of steps and meet the diagonal together), else two consecutive row tiles of one head.  The two
 // tiles ping-pong through the pipeline:
@@ -96,6 +96,11 @@ struct Sm100Dev {
     int item_cost;    // units of the work line that stand for an item's fixed cost (see kItemCostDefault)
     int causal;       // mask type: 0 none, 1 top-left, 2 bottom-right, 3 window with top-left alignment
     int wl, wr;       // window of a masked problem: keys [i + shift - wl, i + shift + wr] of row i; -1 = unbounded
+    // prefill work list: all sequences have the stated lengths (no length arrays); row blocks with a single Q tile behind the
+    // others of a sequence; 2^32 / divisor, rounded up (0: divisor 1), of the items of a row block and of the inner factor
+    // of the order of row blocks (see the schedule in the kernel)
+    int uniform, light;
+    uint32_t inv_per_group, inv_inner;
     int num_levels;   // row blocks of the longest sequence (128 rows when heads are paired, else 256)
     int pair_heads;   // the two Q tiles of a work item are two q heads of one kv group
     float scale_log2;
@@ -330,6 +335,10 @@ constexpr int kMaxLevels = 512;   // row blocks per sequence the on-chip schedul
 constexpr int STAGE_BYTES = 32 * 32 * 2;  // per softmax warp: 32 rows x 32 columns of O on their way to a TMA store
 constexpr int kMaxRounds = 1024;  // work items per CTA (the host sends larger problems to the general instance)
 constexpr int kSplitItems = 2560; // the same for the split modes (their list needs one word per item)
+// Prefill work list: up to kMaxGroups (sequence, row block) pairs are sorted by what they cost; the heads of a pair cost
+// the same, and the last round's items of a grid of at most kDealCtas are dealt by the loads the CTAs have so far.
+constexpr int kMaxGroups = 512;
+constexpr int kDealCtas = 160;
 
 // One work item = two 128-row Q tiles that share their K/V tiles.  With an even GQA ratio the tiles are the same
 // 128 rows of two neighbouring q heads of one kv group: both see the same keys, so they run the same number of
@@ -358,8 +367,10 @@ struct Ctrl {
     int level_start[kMaxLevels + 1];    // first work item of each level; level 0 = highest block index
     int nblk[kMaxBatch];                // row blocks of each sequence
     int seq_q0[kMaxBatch], seq_sq[kMaxBatch], seq_k0[kMaxBatch], seq_sk[kMaxBatch];  // first row / length, Q and K
+    // (prefill: the words behind kMaxRounds hold the sorted groups and the CTAs' loads while the list is made)
     // this CTA's work list: valid << 31 | sequence << 22 | head index << 12 | row block (split modes: split << 4 | block)
-    uint32_t items[kSplitItems];
+    alignas(16) uint32_t items[kSplitItems];
+    int rounds;                         // prefill: items of this CTA
     int split_w, split_items;           // split modes: length of a CTA's piece of the work stream; items of this CTA
     // split modes: every item takes all key tiles of its stream, except that the first item of the list may start
     // inside its stream (at this tile) and the last one may end inside it (before this tile)
@@ -499,12 +510,187 @@ __device__ __forceinline__ void expand_item(const Ctrl* ctrl, const Sm100Dev& p,
     it.N = max(it.nt[0], it.nt[1]);
 }
 
+// What an item of a group costs, in quarters of a two-tile step (3800 clocks; a single tile takes about three quarters of
+// one), with the 4500 clocks an item spends outside its steps.  (A load of kMaxRounds of them stays below 2^23.)
+__device__ __forceinline__ uint32_t group_cost(const Ctrl* ctrl, const Sm100Dev& p, uint32_t packed) {
+    Item it;
+    expand_item(ctrl, p, packed, it);
+    return (uint32_t)min((min(it.nt[0], it.nt[1]) > 0 ? 4 : 3) * it.N + 5, 8191);
+}
+
 // The work item of round `rnd` of this CTA, from the table filled at start-up.
 template <int SPLIT = 0>
 __device__ __forceinline__ void get_item(const Ctrl* ctrl, const Sm100Dev& p, int rnd, int total_items, int lane, Item& it) {
     if (SPLIT) expand_item_split(ctrl, p, ctrl->items[rnd], rnd, it);
     else expand_item(ctrl, p, ctrl->items[rnd], it);
 }
+
+// Fills ctrl->items and ctrl->rounds of a prefill form from the lengths in the control block; every thread calls it, and the
+// caller synchronises afterwards.
+template <bool BIAS>
+__device__ __forceinline__ void prefill_work_list(Ctrl* ctrl, const Sm100Dev& p) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // Prefill schedule.  A group is the items of one (sequence, row block), one per head or pair of heads, which cost the
+    // same.  Three orders of the groups:
+    //   uniform lengths: known in closed form.  With a mask or a bias by decreasing row block (decreasing cost; batches that
+    //     share a bias plane read its rows together: 4 x 5432 tokens 378 us, sequence by sequence 431), otherwise, the costs
+    //     being equal, sequence by sequence, whose blocks read the same K/V.
+    //   sorted: the groups, numbered by sequence and decreasing block, fit a table and are sorted by cost.
+    //   by level: everything else (and a bias with lengths of their own): by decreasing row block.
+    int num_groups = p.batch * p.num_levels;
+    if (!p.uniform) {
+        if (warp == 0) {  // first group of every sequence
+            int run = 0;
+            for (int base = 0; base < p.batch; base += 32) {
+                const int n = base + lane < p.batch ? ctrl->nblk[base + lane] : 0;
+                int incl = n;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, incl, off);
+                    if (lane >= off) incl += y;
+                }
+                if (base + lane < p.batch) ctrl->level_start[base + lane] = run + incl - n;
+                run += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            if (lane == 0) ctrl->level_start[p.batch] = run;
+        }
+        __syncthreads();
+        num_groups = ctrl->level_start[p.batch];
+    }
+    const int per_group = p.pair_heads ? p.hq / 2 : p.hq;
+    auto sequence_of = [&](int g) {  // (lengths of their own) the last sequence whose groups start at or before g
+        int b = 0, bh = p.batch;
+        while (bh - b > 1) {
+            const int mid = (b + bh) >> 1;
+            if (ctrl->level_start[mid] <= g) b = mid; else bh = mid;
+        }
+        return b;
+    };
+    const bool uniform = p.uniform;
+    if (!uniform && num_groups * (int64_t)per_group <= gridDim.x) {  // one item per CTA at most: the order does not matter
+        if (threadIdx.x == 0) {
+            const int g = (int)blockIdx.x / per_group;
+            uint32_t word = 0u;
+            if (g < num_groups) {
+                const int b = sequence_of(g);
+                word = 0x80000000u | ((uint32_t)b << 22) | ((uint32_t)((int)blockIdx.x - g * per_group) << 12) |
+                       (uint32_t)(ctrl->nblk[b] - 1 - (g - ctrl->level_start[b]));
+            }
+            ctrl->items[0] = word;
+            ctrl->rounds = 1;
+        }
+        return;
+    }
+    const bool sorted = !BIAS && !uniform && num_groups <= kMaxGroups;
+    const bool by_level = !uniform && !sorted;
+    uint32_t* const g_key = ctrl->items + kMaxRounds;   // cost << 9 | 511 - number, by number (later: the CTAs' loads)
+    uint32_t* const g_item = g_key + kMaxGroups;        // sequence << 22 | block, in order of decreasing cost
+    uint32_t* const g_cost = g_item + kMaxGroups;
+    static_assert(kMaxRounds + 3 * kMaxGroups <= kSplitItems && kDealCtas <= kMaxGroups && kMaxGroups <= 512, "");
+    if (sorted) {
+#pragma unroll 1
+        for (int g = threadIdx.x; g < num_groups; g += NTHREADS) {
+            const int b = sequence_of(g);
+            const uint32_t group = ((uint32_t)b << 22) | (uint32_t)(ctrl->nblk[b] - 1 - (g - ctrl->level_start[b]));
+            ctrl->items[g] = group;  // (the work list itself comes later)
+            g_key[g] = (group_cost(ctrl, p, group) << 9) | (uint32_t)(511 - g);
+        }
+        if (threadIdx.x < 4 && num_groups + threadIdx.x < kMaxGroups) g_key[num_groups + threadIdx.x] = 0u;
+        __syncthreads();
+#pragma unroll 1
+        for (int g = threadIdx.x; g < num_groups; g += NTHREADS) {  // place = number of larger keys (all are different)
+            const uint32_t key = g_key[g];
+            int place = 0;
+#pragma unroll 4
+            for (int k = 0; k < num_groups; k += 4) {
+                const uint4 o = *reinterpret_cast<const uint4*>(g_key + k);
+                place += (o.x > key) + (o.y > key) + (o.z > key) + (o.w > key);
+            }
+            g_item[place] = ctrl->items[g];
+            g_cost[place] = key >> 9;
+        }
+    }
+    for (int lv = threadIdx.x; by_level && lv < p.num_levels; lv += NTHREADS) {  // count of sequences that have block index lv
+        int c = 0;
+        for (int b = 0; b < p.batch; ++b) c += ctrl->nblk[b] > lv;
+        ctrl->items[lv] = c * per_group;
+    }
+    __syncthreads();
+    if (by_level && threadIdx.x == 0) {
+        int run = 0;
+        ctrl->level_start[0] = 0;
+        for (int lv = 1; lv <= p.num_levels; ++lv) {
+            run += (int)ctrl->items[p.num_levels - lv];
+            ctrl->level_start[lv] = run;
+        }
+    }
+    __syncthreads();
+    const int total_items = by_level ? ctrl->level_start[p.num_levels] : num_groups * per_group;
+    int rounds = (total_items + (int)gridDim.x - 1) / (int)gridDim.x;
+    if (rounds > kMaxRounds) {  // the host checks an upper bound of this; never silently drop work
+        if (threadIdx.x == 0) atomicOr(p.status, FLASHCK_STATUS_WORKLIST_OVERFLOW);
+        rounds = 0;
+    }
+    // This CTA's work list: dealt in snake order, except that the last round's items of a sorted list go, dearest first, to
+    // the CTAs in order of the load they have so far (which evens out a round that is not full, too).  The items of a chunked
+    // prefill differ by their sequences' lengths, up to 60 % of a CTA's whole share: by row block alone the last CTA of six
+    // sequences of 1-16k keys (368 items) had 1.59 times the mean load, now 1.15 times (550 -> 407 us).  Over 150 problems
+    // the mean of last / mean load is 1.21 by row block, 1.16 in snake order over sorted items, 1.142 with one dealt round
+    // and 1.140 with all rounds dealt; a dealt round takes 0.9 us (a chain of a few hundred instructions that are fetched
+    // for it alone), which is why the uniform orders, whose snake is even but for a last round that is not full, have none.
+    if (by_level) {
+        for (int rnd = warp; rnd < rounds; rnd += NTHREADS / 32) {
+            const int w = item_of_round(rnd, blockIdx.x, gridDim.x);
+            const uint32_t packed = w >= total_items ? 0u : find_item(ctrl, p, w, lane);
+            if (lane == 0) ctrl->items[rnd] = packed;
+        }
+    } else {
+        const int g = (int)gridDim.x, j = (int)threadIdx.x;
+        auto div_by = [](int x, uint32_t inv) { return inv ? (int)__umulhi((uint32_t)x, inv) : x; };
+        auto group_item = [&](int gi) -> uint32_t {  // sequence << 22 | row block of group gi
+            if (!uniform) return g_item[gi];
+            const int full = p.num_levels - p.light;  // (blocks of a single tile come last: they are the cheapest)
+            const int outer = div_by(gi, p.inv_inner);
+            if (p.causal || BIAS) return ((uint32_t)(gi - outer * p.batch) << 22) | (uint32_t)(p.num_levels - 1 - outer);
+            if (gi >= p.batch * full) return ((uint32_t)(gi - p.batch * full) << 22) | (uint32_t)full;
+            return ((uint32_t)outer << 22) | (uint32_t)(full - 1 - (gi - outer * full));
+        };
+        auto item_word = [&](int w) -> uint32_t {
+            if (w >= total_items) return 0u;
+            const int gi = div_by(w, p.inv_per_group);
+            return 0x80000000u | group_item(gi) | ((uint32_t)(w - gi * per_group) << 12);
+        };
+        const bool deal = sorted && g <= kDealCtas;
+        const int last = deal ? rounds - 1 : rounds;
+#pragma unroll 1
+        for (int rnd = j; rnd < last; rnd += NTHREADS) ctrl->items[rnd] = item_word(item_of_round(rnd, blockIdx.x, g));
+        if (deal) {
+            if (j < kDealCtas) {
+                uint32_t load = 0u;  // of CTA j
+#pragma unroll 1
+                for (int rnd = 0; j < g && rnd < last; ++rnd) load += g_cost[div_by(item_of_round(rnd, j, g), p.inv_per_group)];
+                g_key[j] = j < g ? (load << 9) | (uint32_t)j : 0xffffffffu;
+            }
+            __syncthreads();
+            // only this CTA's own place matters: the number of smaller keys
+            if (warp == 0) {
+                const uint32_t key = g_key[blockIdx.x];
+                uint32_t n = 0;
+#pragma unroll
+                for (int u = 0; u < kDealCtas / 32; ++u) n += g_key[lane + 32 * u] < key;
+                n = __reduce_add_sync(0xffffffffu, n);
+                if (lane == 0) ctrl->items[last] = item_word(last * g + (int)n);
+            }
+        }
+    }
+    if (threadIdx.x == 0) ctrl->rounds = rounds;
+}
+
+// Out of line its values take no registers from the role loops (104 instead of 128 bytes of reloads: 1006 against 1016 us on
+// 16 x 512-4096 tokens); the bias instances, whose loops came out slower that way (262 against 253 us on 2 x 2048 tokens),
+// keep it inline.
+template <bool BIAS>
+__device__ __noinline__ void prefill_work_list_call(Ctrl* ctrl, const Sm100Dev& p) { prefill_work_list<BIAS>(ctrl, p); }
 
 // VAR bit 1 (EXTRA): the scaled scores get the reference's score additions that need no memory traffic -- a logits soft
 //          cap (cap * tanh(score / cap), core/profiling/attention/fmha_fwd/fmha_fwd_problem.h:81) and ALiBi
@@ -536,7 +722,7 @@ template <typename T, int EXPM, int VAR, int SPLIT, int HDIM = 128>
 __global__ void __launch_bounds__(NTHREADS, 1)
 fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
-                      const Sm100Dev p) {
+                      const __grid_constant__ Sm100Dev p) {
     extern __shared__ uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // head dim of this instance (128, or 64 for the prefill forms): the names below shadow the file-scope constants
@@ -708,13 +894,21 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             ctrl->split_items = cnt;
         }
     }
-    for (int lv = threadIdx.x; !SPLIT && lv < p.num_levels; lv += NTHREADS) {  // count of sequences that have block index lv
+    // The hdim-64 instances keep their items in order of levels, worked out in place: ptxas' allocation in their role loops
+    // moves with the code in front of them, and with the lists above, inline or called, it came out 2-10 % slower (4 x 4096
+    // tokens, 32 heads, no mask: 699 us; called 759, inline 770).
+    constexpr bool LEVELS = SPLIT == 0 && HDIM == 64;
+    if constexpr (SPLIT == 0 && !LEVELS) {
+        if constexpr (BIAS) prefill_work_list<BIAS>(ctrl, p);
+        else prefill_work_list_call<BIAS>(ctrl, p);
+    }
+    for (int lv = threadIdx.x; LEVELS && lv < p.num_levels; lv += NTHREADS) {  // count of sequences that have block index lv
         int c = 0;
         for (int b = 0; b < p.batch; ++b) c += ctrl->nblk[b] > lv;
         ctrl->level_start[p.num_levels - lv] = c * (p.pair_heads ? p.hq / 2 : p.hq);  // summed up below
     }
     __syncthreads();
-    if (!SPLIT && threadIdx.x == 0) {
+    if (LEVELS && threadIdx.x == 0) {
         int run = 0;
         ctrl->level_start[0] = 0;
         for (int lv = 1; lv <= p.num_levels; ++lv) {
@@ -726,13 +920,13 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctrl->tmem_base;
-    const int total_items = SPLIT ? 0 : ctrl->level_start[p.num_levels];
-    int rounds = SPLIT ? ctrl->split_items : (total_items + (int)gridDim.x - 1) / (int)gridDim.x;
-    if (!SPLIT && rounds > kMaxRounds) {  // the host checks an upper bound of this; never silently drop work
+    const int total_items = LEVELS ? ctrl->level_start[p.num_levels] : 0;
+    int rounds = SPLIT ? ctrl->split_items : !LEVELS ? ctrl->rounds : (total_items + (int)gridDim.x - 1) / (int)gridDim.x;
+    if (LEVELS && rounds > kMaxRounds) {  // the host checks an upper bound of this; never silently drop work
         if (threadIdx.x == 0) atomicOr(p.status, FLASHCK_STATUS_WORKLIST_OVERFLOW);
         rounds = 0;
     }
-    for (int rnd = warp; !SPLIT && rnd < rounds; rnd += NTHREADS / 32) {  // this CTA's work list
+    for (int rnd = warp; LEVELS && rnd < rounds; rnd += NTHREADS / 32) {  // this CTA's work list
         const int w = item_of_round(rnd, blockIdx.x, gridDim.x);
         const uint32_t packed = w >= total_items ? 0u : find_item(ctrl, p, w, lane);
         if (lane == 0) ctrl->items[rnd] = packed;
@@ -1673,6 +1867,14 @@ int launch_fwd_sm100(const FwdParams& p, cudaStream_t stream) {
     dev.wr = p.wr < 0 ? -1 : (int)p.wr;
     dev.pair_heads = ((p.hq / p.hkv) % 2 == 0) ? 1 : 0;
     dev.num_levels = (int)((p.max_seqlen_q + (dev.pair_heads ? BM : 2 * BM) - 1) / (dev.pair_heads ? BM : 2 * BM));
+    {   // the work list (see the schedule in the kernel)
+        const auto inverse = [](int64_t d) { return d > 1 ? (uint32_t)(((1ll << 32) + d - 1) / d) : 0u; };
+        dev.uniform = !p.seqstart_q && !p.seqstart_k && !p.kv_indptr && !p.seqlen_k32;
+        // (without a pair of heads a block is two row tiles: an odd number of tiles leaves a last block of one)
+        dev.light = !dev.pair_heads && ((p.max_seqlen_q + BM - 1) / BM) % 2 != 0 ? 1 : 0;
+        dev.inv_per_group = inverse(dev.pair_heads ? p.hq / 2 : p.hq);
+        dev.inv_inner = inverse(p.mask_type != 0 || (p.bias && p.bias_type == 1) ? p.batch : dev.num_levels - dev.light);
+    }
     dev.scale_log2 = p.scale * 1.4426950408889634f;
     const bool bf16 = p.dtype == FLASHCK_DTYPE_BFLOAT16;
     const bool window = p.mask_type != 0 && !(p.wl < 0 && p.wr == 0);

@@ -1,0 +1,46 @@
+"""The prefill kernel's work list: every query row of every sequence is computed once, whichever way the list is made."""
+import pytest
+import torch
+
+from flashck_b200 import _lib, ops
+from flashck_b200.utils.inputs import to_seqstarts, uniform_seqlens
+from tests.helpers import assert_lse_close, assert_o_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, k, v, nq, nk, causal):
+    o, lse, group = torch.empty(q.shape, device=q.device), torch.empty((q.shape[1], q.shape[0]), device=q.device), q.shape[1] // k.shape[1]
+    a = c = 0
+    for n, m in zip(nq, nk):
+        kk, vv = (t[c:c + m].float().repeat_interleave(group, 1) for t in (k, v))
+        x = torch.einsum("qhd,khd->hqk", q[a:a + n].float(), kk) * q.shape[2] ** -0.5
+        if causal:
+            x.masked_fill_(torch.arange(m, device=q.device) > torch.arange(n, device=q.device)[:, None] + (m - n), float("-inf"))
+        lse[:, a:a + n] = torch.logsumexp(x, -1)
+        o[a:a + n] = torch.einsum("hqk,khd->qhd", torch.softmax(x, -1), vv)
+        a, c = a + n, c + m
+    return o, lse
+
+
+# batch, longest query, heads: a handful of items; lists dealt by load (2-16 rounds); 511 - 513 row blocks, the edge of the
+# sorted table; one block per sequence at the largest batch; more than 16 rounds in snake order; far more row blocks than
+# the table holds
+@pytest.mark.parametrize("batch,lo,hi,hq,hkv", [
+    (1, 1, 1, 8, 8), (3, 1, 700, 8, 2), (37, 1, 900, 8, 2), (37, 1, 900, 12, 4), (256, 1, 128, 4, 2),
+    (256, 129, 256, 2, 1), (171, 257, 384, 2, 1), (170, 257, 384, 6, 2), (64, 900, 1000, 12, 4), (64, 900, 1000, 12, 2), (250, 300, 500, 8, 2),
+])
+@pytest.mark.parametrize("causal,more", [(True, 0), (False, 0), (True, 1500)])
+def test_every_row_once(batch, lo, hi, hq, hkv, causal, more):
+    if more and batch > 40:
+        pytest.skip("(the mask and the list do not depend on both)")
+    nq = uniform_seqlens(batch, lo, hi, batch + hi)
+    nk = [n + e for n, e in zip(nq, uniform_seqlens(batch, 0, more, 3))] if more else nq
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    q, k, v = (torch.randn((sum(n), h, 128), generator=g, device="cuda").bfloat16() for n, h in ((nq, hq), (nk, hkv), (nk, hkv)))
+    cu_q, cu_k = to_seqstarts(nq).cuda(), to_seqstarts(nk).cuda()
+    o, lse = ops.fmha_fwd_var_len(q, k, v, cu_q, cu_k, max(nq), causal=causal, return_lse=True)
+    assert _lib.device_status() == 0
+    o_ref, lse_ref = _reference(q, k, v, nq, nk, causal)
+    assert_o_close(o, o_ref)
+    assert_lse_close(lse, lse_ref)
