@@ -13,6 +13,7 @@ functions take packed ``[total, h, d]`` tensors plus ``cu_seqlens`` (int64 ``[b+
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from typing import Optional, Sequence, Tuple
 
@@ -61,12 +62,21 @@ def _check_cuda(name: str, t: Optional[torch.Tensor], dtype=None) -> None:
         raise TypeError(f"{name} must have dtype {dtype}, got {t.dtype}")
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+# Pointers travel as plain integers (the bound signatures convert them), and the device is only switched when it is another
+# one: around a short call these wrappers took longer than its kernels.
+def _ptr(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    return torch.cuda.current_stream().cuda_stream
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def _mask(causal: bool, window_size: Sequence[int], mask_type: Optional[int]) -> Tuple[int, int, int]:
@@ -107,7 +117,7 @@ def _alibi_args(alibi_slopes: Optional[torch.Tensor], batch: int, hq: int):
     kind of bias per call (ALiBi slopes fp32 ``[1|batch, hq]`` or nothing), so that no process-wide instance parameter
     is touched on the launch path."""
     if alibi_slopes is None:
-        return ctypes.c_void_p(0), 0, 0
+        return 0, 0, 0
     _check_cuda("alibi_slopes", alibi_slopes, torch.float32)
     if alibi_slopes.dim() != 2 or alibi_slopes.shape[1] != hq or alibi_slopes.shape[0] not in (1, batch):
         raise ValueError(f"alibi_slopes must be fp32 [1|{batch}, {hq}], got {tuple(alibi_slopes.shape)}")
@@ -183,7 +193,7 @@ def fmha_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: Option
     o = torch.empty((b, sq, hq, dv), dtype=q.dtype, device=q.device)
     lse = torch.empty((b, hq, sq), dtype=torch.float32, device=q.device) if return_lse else None
     bias_buf, bias_enum, bias_rank = _bias_args(q, bias, alibi_slopes, b, hq, sq, sk)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         rc = _launch_tuned(
             "fmha_fwd", dict(dtype=_dtype_name(q), mode="batch", batch=b, hq=hq, hkv=hkv, d=d, dv=dv, max_seqlen_q=sq,
                              max_seqlen_k=sk, mask=_mask_name(mt, wl, wr), bias=("none", "elementwise", "alibi")[bias_enum],
@@ -248,7 +258,7 @@ def fmha_fwd_fp8(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale_s: 
     mt, wl, wr = _mask(causal, window_size, mask_type)
     o = torch.empty(o_shape + (dv,), dtype=out_dtype, device=q.device)
     lse = torch.empty(lse_shape, dtype=torch.float32, device=q.device) if return_lse else None
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         rc = _lib.lib().FmhaFwdFp8(_ptr(q), _ptr(k), _ptr(v), _ptr(o), _ptr(cu_q), _ptr(cu_k), batch, sq, sk, hq, hkv, d, dv,
                                    max_sq, float(scale_s), float(scale_p), float(scale_o), wl, wr, mt, _stream(), _ptr(lse),
                                    code, out_code)
@@ -286,7 +296,7 @@ def fmha_fwd_var_len(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqle
     lse = torch.empty((hq, total_q), dtype=torch.float32, device=q.device) if return_lse else None
     bias_buf, bias_enum, bias_rank = _bias_args(q, bias, alibi_slopes, 1 if bias is not None else batch, hq, total_q,
                                                 total_k)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         rc = _launch_tuned(
             "fmha_fwd", dict(dtype=_dtype_name(q), mode="group", batch=batch, hq=hq, hkv=hkv, d=d, dv=dv,
                              max_seqlen_q=int(max_seqlen_q), max_seqlen_k=int(max_seqlen_k) or int(max_seqlen_q),
@@ -330,7 +340,7 @@ def batch_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, c
     o = torch.empty((total_q, hq, dv), dtype=q.dtype, device=q.device)
     lse = torch.empty((hq, total_q), dtype=torch.float32, device=q.device) if return_lse else None
     bias_ptr, bias_enum, bias_rank = _alibi_args(alibi_slopes, batch, hq)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         rc = _lib.lib().FmhaFwdBatchPrefillEx(_ptr(q), _ptr(k_pool), _ptr(v_pool), bias_ptr, _ptr(o), _ptr(cu_q),
                                               _ptr(indptr), _ptr(indices), _ptr(last), batch, total_q, hq, hkv, d, dv,
                                               int(max_seqlen_q), pages, page, float(scale or 0.0), wl, wr, mt,
@@ -375,7 +385,7 @@ def fmha_fwd_paged_kv_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
     o = torch.empty(o_shape + (dv,), dtype=q.dtype, device=q.device)
     lse = torch.empty(lse_shape, dtype=torch.float32, device=q.device) if return_lse else None
     bias_ptr, bias_enum, bias_rank = _alibi_args(alibi_slopes, batch, hq)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         rc = _lib.lib().FmhaFwdPagedKVPrefillEx(_ptr(q), _ptr(k_pool), _ptr(v_pool), bias_ptr, _ptr(o), _ptr(cu_q),
                                                 _ptr(sl), _ptr(bt), _ptr(cbi), batch, shape_sq, hq, hkv, d, dv, max_sq,
                                                 batch * bt.shape[1], page, float(scale or 0.0), wl, wr, mt, _stream(),
@@ -445,7 +455,7 @@ def fmha_fwd_splitkv_combine(lse_acc: torch.Tensor, o_acc: torch.Tensor, dtype: 
     lse = lse_out if lse_out is not None else (
         torch.empty((bs, hq, rows), dtype=torch.float32, device=o_acc.device) if return_lse else None)
     _check_cuda("lse_out", lse, torch.float32)
-    with torch.cuda.device(o_acc.device):
+    with _on(o_acc.device):
         if dtype == torch.float32:
             ls = (ctypes.c_int64 * 4)(hq * S * rows, S * rows, rows, 1)
             os_ = (ctypes.c_int64 * 4)(hq * S * rows * dv, S * rows * dv, rows * dv, dv)
@@ -477,7 +487,7 @@ def fmha_fwd_splitkv_combine_strided(buf: torch.Tensor, batch: int, rows: int, h
     lse = torch.empty((batch, hq, rows), dtype=torch.float32, device=buf.device) if return_lse else None
     ls = (ctypes.c_int64 * 4)(*[int(x) for x in lse_strides])
     os_ = (ctypes.c_int64 * 4)(*[int(x) for x in o_strides])
-    with torch.cuda.device(buf.device):
+    with _on(buf.device):
         rc = _lib.lib().FmhaFwdSplitKVCombineStrided(ctypes.c_void_p(buf.data_ptr() + 4 * int(lse_offset)), _ptr(buf),
                                                      _ptr(o), _ptr(lse), batch, rows, hq, dv, num_splits, ls, os_, code,
                                                      _stream())
@@ -547,7 +557,7 @@ def fmha_fwd_splitkv(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     # pages of a paged pool, or rows of a contiguous cache (packed K/V: unused): where the K/V tensor maps end
     pool_extent = 0 if cu_k is not None else k_cache.shape[0]
     cap_k = bt.shape[1] * page if bt is not None else shape_sk
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         rc = _launch_tuned(
             "fmha_fwd_split_kv", dict(dtype=_dtype_name(q), mode="group" if group else "batch", batch=batch, hq=hq, hkv=hkv,
                                       d=d, dv=dv, max_seqlen_q=max_sq, max_seqlen_k=int(cap_k), mask=_mask_name(mt, wl, wr),
@@ -610,7 +620,7 @@ def fmha_fwd_append_kv(q: Optional[torch.Tensor], k_cache: torch.Tensor, v_cache
         page, max_pages, cap = k_cache.shape[1], batch * bt.shape[1], 0
     else:
         page, max_pages, cap = 0, 0, k_cache.shape[1]
-    with torch.cuda.device(k_cache.device):
+    with _on(k_cache.device):
         rc = _lib.lib().FmhaFwdAppendKV(_ptr(q), _ptr(k_cache), _ptr(knew), _ptr(v_cache), _ptr(vnew), _ptr(sl),
                                         _ptr(cu_q), _ptr(cu_n), _ptr(rotary_cos), _ptr(rotary_sin), _ptr(bt),
                                         _ptr(cbi), batch, sq, cap, n_new, hq, hkv, d, dv, int(rotary_dim), rope,
