@@ -239,8 +239,8 @@ __device__ __forceinline__ void soft_cap_scores(uint32_t* s, float scale_log2, f
         asm("{\n.reg .f32 a, b;\nabs.f32 a, %1;\nabs.f32 b, %2;\nmax.f32 %0, %0, a, b;\n}\n" : "+f"(a0) : "r"(s[j]), "r"(s[j + 1]));
         asm("{\n.reg .f32 a, b;\nabs.f32 a, %1;\nabs.f32 b, %2;\nmax.f32 %0, %0, a, b;\n}\n" : "+f"(a1) : "r"(s[j + 2]), "r"(s[j + 3]));
     }
-    // (a k beyond 1e3 could overflow its eighth power; a NaN passes either way)
-    if (__all_sync(0xffffffffu, fmaxf(a0, a1) * k <= 0.5f && k < 1e3f)) {
+    // (a negative scale makes k negative; a k beyond 1e3 could overflow its eighth power; a NaN passes either way)
+    if (__all_sync(0xffffffffu, fmaxf(a0, a1) * fabsf(k) <= 0.5f && fabsf(k) < 1e3f)) {
         const float k2 = k * k, c0 = scale_log2, c1 = -0.33333069f * (c0 * k2), c2 = 0.13324779f * (c0 * k2 * k2),
                     c3 = -0.052986056f * (c0 * k2 * k2 * k2), c4 = 0.017135002f * (c0 * (k2 * k2) * (k2 * k2));
 #pragma unroll

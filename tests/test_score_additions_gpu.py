@@ -51,3 +51,29 @@ def test_score_additions(size, d, n, m, add, causal, window):
     o_ref, lse_ref = _reference(q, k, v, causal, window, cap, slopes, bias)
     assert_o_close(o, o_ref)
     assert_lse_close(lse, lse_ref)
+
+
+# The polynomial holds for |score| <= cap / 2 whichever sign the scale has; scores here reach three caps and more.
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("add", ["cap", "cap+alibi", "cap+bias"])
+@pytest.mark.parametrize("packed", [False, True])
+def test_soft_cap_with_a_negative_scale(d, add, packed):
+    n, m, cap, scale = 300, 300, 20.0, -d ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, k, v = (torch.randn((2, s, h, d), generator=g, device="cuda").bfloat16() for s, h in ((n, 6), (m, 2), (m, 2)))
+    q = q * 20
+    slopes = (2.0 ** -torch.arange(1, 7, device="cuda").float())[None] if "alibi" in add else None
+    bias = torch.randn((1, 6, n, m), generator=g, device="cuda").bfloat16() if "bias" in add else None
+    more = dict(causal=True, scale=scale, logits_soft_cap=cap, alibi_slopes=slopes, return_lse=True)
+    if packed:
+        cu = torch.tensor([0, n, 2 * n], device="cuda")
+        if bias is not None:  # (packed: one plane over the packed totals)
+            more["bias"] = torch.nn.functional.pad(torch.cat([bias, bias], 2), (0, m))
+            more["bias"][:, :, n:, m:] = bias
+        o, lse = ops.fmha_fwd_var_len(q.flatten(0, 1), k.flatten(0, 1), v.flatten(0, 1), cu, cu, n, **more)
+        o, lse = o.view(2, n, 6, d), lse.view(6, 2, n).transpose(0, 1)
+    else:
+        o, lse = ops.fmha_fwd(q, k, v, bias=bias, **more)
+    o_ref, lse_ref = _reference(-q, k, v, True, -1, cap, slopes, bias)
+    assert_o_close(o, o_ref)
+    assert_lse_close(lse, lse_ref)
