@@ -71,6 +71,13 @@ std::atomic<int64_t> g_exp_mode{0};
 std::atomic<int64_t> g_exp_mode_splitkv{0};
 std::atomic<int64_t> g_use_sm100_splitkv{1};  // multi-token split-KV on the tcgen05 instance
 
+// Constants of the logits soft cap (soft_cap_scores), from the scale and the cap.
+struct SoftCap {
+    float lim;                 // raw scores up to this magnitude take the polynomial
+    float c0, c1, c2, c3, c4;  // its coefficients in powers of the squared raw score
+    float k2e, c, m2c;         // the quotient form: exponent per unit of raw score, cap in base-2 units, -2 c
+};
+
 struct Sm100Dev {
     void* o;
     float* lse;
@@ -104,8 +111,8 @@ struct Sm100Dev {
     int num_levels;   // row blocks of the longest sequence (128 rows when heads are paired, else 256)
     int pair_heads;   // the two Q tiles of a work item are two q heads of one kv group
     float scale_log2;
-    float scale;            // EXTRA instances: the softmax scale itself
     float soft_cap;         // EXTRA: 0 = off
+    SoftCap cap;            // EXTRA with soft_cap > 0
     const float* alibi;     // EXTRA: fp32 slopes [1,hq] (alibi_rank 0) or [batch,hq] (1), or nullptr
     int alibi_rank;
     float rescale_thr;  // the running max is raised (and O rescaled) when the row max exceeds it by more than this (log2 units)
@@ -226,39 +233,61 @@ __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.p
 
 // Logits soft cap on N raw scores of one row: s -> cap * tanh(s * k) * log2(e), k = scale / cap, in place.  Three operations
 // of the exp2 unit per element (the exponential and the reciprocal of tanh, then the softmax's own exponential) keep that
-// unit busy three times as long as the rest of the softmax takes.  Where every score of the warp is within half a cap,
-// tanh(y) is y * P(y^2) instead, P the polynomial of degree 4 that fits tanh(y) / y on [0, 0.5] best in relative error
-// (1.3e-8; 1.1e-7 with its fp32 rounding, against 1.5e-4 near 0 of the quotient form): with the scale folded into the
-// coefficients six packed operations per pair of elements.  2 x 5000 tokens, 32 heads, window 1023: 453 -> 257 us; causal
-// without a window 1032 -> 512; hdim 64, 4 x 4096 without a mask, cap 50: 2546 -> 1310.
+// unit busy three times as long as the rest of the softmax takes.  A score within half a cap takes tanh(y) = y * P(y^2)
+// instead, P the polynomial of degree 4 in y^2 that fits tanh(y) / y on [0, 0.5] in relative error (2.9e-8; 1.5e-7 with its
+// fp32 rounding, where the quotient form loses up to 1.5e-4 near 0): with the scale folded into the coefficients six packed
+// operations per pair of elements, and where all scores of the warp are that small nothing else.  A warp with a larger score
+// works out both forms and picks per score, so that a score's value depends on that score alone.
+// us with the quotient form for every score / scores up to 0.4 caps / up to 3 caps: 2 x 5000 tokens, 32 heads, window 1023,
+// 453 / 240 / 399; hdim 64, 4 x 4096 causal, 1322 / 620 / 1184; 2 x 4096 without a mask, 1294 / 619 / 1135; causal with ALiBi,
+// 688 / 432 / 680.
 template <int N>
-__device__ __forceinline__ void soft_cap_scores(uint32_t* s, float scale_log2, float cap, float k) {
+__device__ __forceinline__ void soft_cap_scores(uint32_t* s, const SoftCap& p) {
     float a0 = 0.f, a1 = 0.f;
 #pragma unroll
     for (int j = 0; j < N; j += 4) {
         asm("{\n.reg .f32 a, b;\nabs.f32 a, %1;\nabs.f32 b, %2;\nmax.f32 %0, %0, a, b;\n}\n" : "+f"(a0) : "r"(s[j]), "r"(s[j + 1]));
         asm("{\n.reg .f32 a, b;\nabs.f32 a, %1;\nabs.f32 b, %2;\nmax.f32 %0, %0, a, b;\n}\n" : "+f"(a1) : "r"(s[j + 2]), "r"(s[j + 3]));
     }
-    // (a negative scale makes k negative; a k beyond 1e3 could overflow its eighth power; a NaN passes either way)
-    if (__all_sync(0xffffffffu, fmaxf(a0, a1) * fabsf(k) <= 0.5f && fabsf(k) < 1e3f)) {
-        const float k2 = k * k, c0 = scale_log2, c1 = -0.33333069f * (c0 * k2), c2 = 0.13324779f * (c0 * k2 * k2),
-                    c3 = -0.052986056f * (c0 * k2 * k2 * k2), c4 = 0.017135002f * (c0 * (k2 * k2) * (k2 * k2));
+    auto poly = [&](float2 x) {
+        const float2 v = __fmul2_rn(x, x);
+        float2 q = __ffma2_rn(make_float2(p.c4, p.c4), v, make_float2(p.c3, p.c3));
+        q = __ffma2_rn(q, v, make_float2(p.c2, p.c2));
+        q = __ffma2_rn(q, v, make_float2(p.c1, p.c1));
+        q = __ffma2_rn(q, v, make_float2(p.c0, p.c0));
+        return __fmul2_rn(q, x);
+    };
+    if (__all_sync(0xffffffffu, fmaxf(a0, a1) <= p.lim)) {  // (a NaN passes: it stays one either way)
 #pragma unroll
         for (int j = 0; j < N; j += 2) {
-            const float2 x = make_float2(__uint_as_float(s[j]), __uint_as_float(s[j + 1]));
-            const float2 v = __fmul2_rn(x, x);
-            float2 q = __ffma2_rn(make_float2(c4, c4), v, make_float2(c3, c3));
-            q = __ffma2_rn(q, v, make_float2(c2, c2));
-            q = __ffma2_rn(q, v, make_float2(c1, c1));
-            q = __ffma2_rn(q, v, make_float2(c0, c0));
-            q = __fmul2_rn(q, x);
+            const float2 q = poly(make_float2(__uint_as_float(s[j]), __uint_as_float(s[j + 1])));
             s[j] = __float_as_uint(q.x);
             s[j + 1] = __float_as_uint(q.y);
         }
     } else {
-        const float c = cap * kLog2e;
+        // Which branch the warp takes must not show in the result (a row would depend on scores that it does not see): every
+        // score takes the form of its own size here.
+        auto pick = [&](float x, float q, float t) {  // the polynomial, or t with the sign of x
+            uint32_t r;
+            asm("{\n.reg .pred p;\n.reg .f32 a;\n.reg .b32 b;\nabs.f32 a, %1;\nsetp.le.f32 p, a, %4;\n"
+                "lop3.b32 b, %3, %1, 0x80000000, 0x78;\nselp.b32 %0, %2, b, p;\n}\n"
+                : "=r"(r) : "r"(__float_as_uint(x)), "r"(__float_as_uint(q)), "r"(__float_as_uint(t)), "f"(p.lim));
+            return r;
+        };
 #pragma unroll
-        for (int j = 0; j < N; ++j) s[j] = __float_as_uint(c * tanh_inline(__uint_as_float(s[j]) * k));
+        for (int j = 0; j < N; j += 2) {
+            const float2 x = make_float2(__uint_as_float(s[j]), __uint_as_float(s[j + 1]));
+            const float2 q = poly(x), y = __fmul2_rn(x, make_float2(p.k2e, p.k2e));
+            float2 r;
+            asm("{\n.reg .f32 a;\nabs.f32 a, %1;\nex2.approx.ftz.f32 %0, a;\n}\n" : "=f"(r.x) : "f"(y.x));
+            asm("{\n.reg .f32 a;\nabs.f32 a, %1;\nex2.approx.ftz.f32 %0, a;\n}\n" : "=f"(r.y) : "f"(y.y));
+            r = __fadd2_rn(r, make_float2(1.f, 1.f));
+            asm("rcp.approx.ftz.f32 %0, %0;\n" : "+f"(r.x));
+            asm("rcp.approx.ftz.f32 %0, %0;\n" : "+f"(r.y));
+            const float2 t = __ffma2_rn(make_float2(p.m2c, p.m2c), r, make_float2(p.c, p.c));
+            s[j] = pick(x.x, q.x, t.x);
+            s[j + 1] = pick(x.y, q.y, t.y);
+        }
     }
 }
 
@@ -1438,7 +1467,6 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 const uint32_t tSb = SPLIT ? lane_addr + sb * 128 : tS;
                 const int key0 = (it.n0 + n) * BN + khalf * 64;
                 [[maybe_unused]] const bool capped = EXTRA && p.soft_cap > 0.f;
-                [[maybe_unused]] const float inv_cap = capped ? 1.f / p.soft_cap : 0.f;
                 [[maybe_unused]] uint4 bw[BIAS ? 16 : 1];  // the 128 bias values of this thread's row and key tile
                 if constexpr (BIAS) {  // (issued before the wait for S)
 #pragma unroll
@@ -1463,7 +1491,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     for (int c = 0; c < 4; ++c) {
                         tmem_ld32(tSb + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&sreg[c * 32]));
                         tmem_wait_ld();
-                        if (capped) soft_cap_scores<32>(&sreg[c * 32], p.scale_log2, p.soft_cap, p.scale * inv_cap);
+                        if (capped) soft_cap_scores<32>(&sreg[c * 32], p.cap);
                         const float mul = capped ? 1.f : p.scale_log2;  // (the two products of the sum in base-2 units)
 #pragma unroll
                         for (int j = 0; j < 32; j += 2) {
@@ -1485,7 +1513,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 if constexpr (EXTRA && !BIAS) {
                     // score additions on the raw scores, before the mask (which must leave -inf behind): the registers
                     // then hold the finished scores in base-2 units, and the scale below becomes 1
-                    if (capped) soft_cap_scores<NC>(sreg, p.scale_log2, p.soft_cap, p.scale * inv_cap);
+                    if (capped) soft_cap_scores<NC>(sreg, p.cap);
                     if (!capped || p.alibi) {
                         const float slope_l2 = slope * kLog2e, mul = capped ? 1.f : p.scale_log2;
                         const float dist0 = (float)(row + sk - sq - key0);  // i + sk - sq - j at the first column
@@ -1939,7 +1967,16 @@ int launch_fwd_sm100(const FwdParams& p, cudaStream_t stream) {
     const bool extra = (p.bias && p.bias_type == 2) || p.logits_soft_cap > 0.f;
     const int expm = extra ? 0 : (int)g_exp_mode.load();
     dev.rescale_thr = expm == 1 ? 0.01f * (float)g_rescale_half_x100.load() : kRescaleThreshold;
-    dev.scale = p.scale; dev.soft_cap = p.logits_soft_cap;
+    dev.soft_cap = p.logits_soft_cap;
+    if (p.logits_soft_cap > 0.f) {
+        const float k = p.scale * (1.f / p.logits_soft_cap), k2 = k * k, c0 = dev.scale_log2;
+        SoftCap& s = dev.cap;
+        // (beyond 1e3 the eighth power of k could overflow)
+        s.lim = fabsf(k) < 1e3f ? 0.5f / fabsf(k) : -1.f;
+        s.c0 = c0; s.c1 = -0.33333069f * (c0 * k2); s.c2 = 0.13324779f * (c0 * k2 * k2);
+        s.c3 = -0.052986056f * (c0 * k2 * k2 * k2); s.c4 = 0.017135002f * (c0 * (k2 * k2) * (k2 * k2));
+        s.k2e = 2.885390081777927f * k; s.c = copysignf(p.logits_soft_cap * kLog2e, k); s.m2c = -2.f * s.c;
+    }
     dev.alibi = (p.bias && p.bias_type == 2) ? (const float*)p.bias : nullptr; dev.alibi_rank = p.bias_rank;
     if (p.dtype == FLASHCK_DTYPE_FLOAT8 || p.dtype == FLASHCK_DTYPE_BFLOAT8) {
         // The running max may lag the row max by `thr` (P up to 2^thr) only as far as P * scale_p stays inside the 8-bit

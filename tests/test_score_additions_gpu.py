@@ -77,3 +77,59 @@ def test_soft_cap_with_a_negative_scale(d, add, packed):
     o_ref, lse_ref = _reference(-q, k, v, True, -1, cap, slopes, bias)
     assert_o_close(o, o_ref)
     assert_lse_close(lse, lse_ref)
+
+
+# What a row computes depends on nothing but the row and the keys it sees: not on the form that the other scores of its warp
+# or its tile ask for.  Changed here: keys that are masked for a row, other rows, the packed sequence behind.
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("add", ["cap", "cap+alibi", "cap+bias"])
+def test_capped_rows_are_independent(d, add):
+    n, cap, cut = 300, 20.0, 203
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, k, v = (torch.randn((1, n, h, d), generator=g, device="cuda").bfloat16() for h in (6, 2, 2))
+    slopes = (2.0 ** -torch.arange(1, 7, device="cuda").float())[None] if "alibi" in add else None
+    bias = torch.randn((1, 6, n, n), generator=g, device="cuda").bfloat16() if "bias" in add else None
+    more = dict(causal=True, logits_soft_cap=cap, alibi_slopes=slopes, return_lse=True)
+    o, lse = ops.fmha_fwd(q, k, v, bias=bias, **more)
+    # later tokens whose scores lie far beyond the cap, as queries and as keys
+    q2, k2 = q.clone(), k.clone()
+    q2[:, cut:] *= 30
+    k2[:, cut:] *= 30
+    o2, lse2 = ops.fmha_fwd(q2, k2, v, bias=bias, **more)
+    assert torch.equal(o2[:, :cut], o[:, :cut]) and torch.equal(lse2[:, :, :cut], lse[:, :, :cut])
+    # single rows in the middle of the warps
+    q3 = q.clone()
+    q3[:, 7::16] *= 30
+    same = torch.arange(n, device="cuda") % 16 != 7
+    o3, lse3 = ops.fmha_fwd(q3, k, v, bias=bias, **more)
+    assert torch.equal(o3[:, same], o[:, same]) and torch.equal(lse3[:, :, same], lse[:, :, same])
+    if bias is None:  # two packed sequences, the second one changed
+        cu = torch.tensor([0, cut, n], device="cuda")
+        a, la = ops.fmha_fwd_var_len(q[0], k[0], v[0], cu, cu, cut, **more)
+        b, lb = ops.fmha_fwd_var_len(q2[0], k2[0], v[0], cu, cu, cut, **more)
+        assert torch.equal(a[:cut], b[:cut]) and torch.equal(la[:, :cut], lb[:, :cut])
+
+
+# One key per sequence and one channel in use: the LSE of a row is its capped score, and the score is exact before the cap.
+# Queries of all sizes from 1e-3 to 4 caps stand side by side in a warp, or each size in warps of its own.
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("scale", [0.0884, 1.0, -0.0884])
+@pytest.mark.parametrize("cap", [0.05, 1.0, 20.0, 900.0])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_capped_score_in_fp32(d, scale, cap, mixed):
+    n = 512
+    x = torch.logspace(-3, 0.6, n, dtype=torch.float64, device="cuda") * (cap / scale)
+    x[::2] *= -1
+    if mixed:
+        x = x[torch.randperm(n, generator=torch.Generator().manual_seed(3)).cuda()]
+    q = torch.zeros((1, n, 2, d), dtype=torch.bfloat16, device="cuda")
+    q[0, :, :, 0] = x.bfloat16()[:, None]
+    k = torch.zeros((1, 1, 2, d), dtype=torch.bfloat16, device="cuda")
+    k[0, 0, :, 0] = 1.0
+    _, lse = ops.fmha_fwd(q, k, k, scale=scale, logits_soft_cap=cap, return_lse=True)
+    s32 = float(torch.tensor(scale)), float(torch.tensor(cap))
+    ref = s32[1] * torch.tanh(q[0, :, :, 0].double().T * s32[0] / s32[1])
+    # polynomial: 3e-8 of its own and about 8 roundings; quotient: 2^-22 of its exponential, twice that at most in 1 - e with
+    # e <= 1 / e, the roundings of the exponent (<= 8 * 2^-24 of a term below 0.6) and of the division; then the LSE's two
+    rel = ((lse[0].double() - ref) / ref).abs().max()
+    assert float(rel) <= 24 * 2.0 ** -24, float(rel)
