@@ -73,8 +73,10 @@ std::atomic<int64_t> g_use_sm100_splitkv{1};  // multi-token split-KV on the tcg
 
 // Constants of the logits soft cap (soft_cap_scores), from the scale and the cap.
 struct SoftCap {
+    float lim_all;             // a warp whose raw scores are all up to this magnitude takes the polynomial and nothing else
     float lim;                 // raw scores up to this magnitude take the polynomial
-    float c0, c1, c2, c3, c4;  // its coefficients in powers of the squared raw score
+    float k;                   // scale / cap: the polynomial's variable is the square of the raw score, or of k times it (lim_all < 0)
+    float c0, c1, c2, c3, c4;  // its coefficients
     float k2e, c, m2c;         // the quotient form: exponent per unit of raw score, cap in base-2 units, -2 c
 };
 
@@ -239,8 +241,8 @@ __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.p
 // operations per pair of elements, and where all scores of the warp are that small nothing else.  A warp with a larger score
 // works out both forms and picks per score, so that a score's value depends on that score alone.
 // us with the quotient form for every score / scores up to 0.4 caps / up to 3 caps: 2 x 5000 tokens, 32 heads, window 1023,
-// 453 / 240 / 399; hdim 64, 4 x 4096 causal, 1322 / 620 / 1184; 2 x 4096 without a mask, 1294 / 619 / 1135; causal with ALiBi,
-// 688 / 432 / 680.
+// 453 / 237 / 411; hdim 64, 4 x 4096 causal, 1322 / 608 / 1190; 2 x 4096 without a mask, 1294 / 604 / 1115; causal with ALiBi,
+// 688 / 421 / 671; 2 x 2048 with a bias per head, 328 / 254 / 338.
 template <int N>
 __device__ __forceinline__ void soft_cap_scores(uint32_t* s, const SoftCap& p) {
     float a0 = 0.f, a1 = 0.f;
@@ -249,18 +251,18 @@ __device__ __forceinline__ void soft_cap_scores(uint32_t* s, const SoftCap& p) {
         asm("{\n.reg .f32 a, b;\nabs.f32 a, %1;\nabs.f32 b, %2;\nmax.f32 %0, %0, a, b;\n}\n" : "+f"(a0) : "r"(s[j]), "r"(s[j + 1]));
         asm("{\n.reg .f32 a, b;\nabs.f32 a, %1;\nabs.f32 b, %2;\nmax.f32 %0, %0, a, b;\n}\n" : "+f"(a1) : "r"(s[j + 2]), "r"(s[j + 3]));
     }
-    auto poly = [&](float2 x) {
-        const float2 v = __fmul2_rn(x, x);
+    auto poly = [&](float2 x, float2 z) {
+        const float2 v = __fmul2_rn(z, z);
         float2 q = __ffma2_rn(make_float2(p.c4, p.c4), v, make_float2(p.c3, p.c3));
         q = __ffma2_rn(q, v, make_float2(p.c2, p.c2));
         q = __ffma2_rn(q, v, make_float2(p.c1, p.c1));
         q = __ffma2_rn(q, v, make_float2(p.c0, p.c0));
         return __fmul2_rn(q, x);
     };
-    if (__all_sync(0xffffffffu, fmaxf(a0, a1) <= p.lim)) {  // (a NaN passes: it stays one either way)
+    if (__all_sync(0xffffffffu, fmaxf(a0, a1) <= p.lim_all)) {  // (a NaN passes: it stays one either way)
 #pragma unroll
         for (int j = 0; j < N; j += 2) {
-            const float2 q = poly(make_float2(__uint_as_float(s[j]), __uint_as_float(s[j + 1])));
+            const float2 x = make_float2(__uint_as_float(s[j]), __uint_as_float(s[j + 1])), q = poly(x, x);
             s[j] = __float_as_uint(q.x);
             s[j + 1] = __float_as_uint(q.y);
         }
@@ -274,20 +276,25 @@ __device__ __forceinline__ void soft_cap_scores(uint32_t* s, const SoftCap& p) {
                 : "=r"(r) : "r"(__float_as_uint(x)), "r"(__float_as_uint(q)), "r"(__float_as_uint(t)), "f"(p.lim));
             return r;
         };
+        auto both = [&](auto powers_tag) {
 #pragma unroll
-        for (int j = 0; j < N; j += 2) {
-            const float2 x = make_float2(__uint_as_float(s[j]), __uint_as_float(s[j + 1]));
-            const float2 q = poly(x), y = __fmul2_rn(x, make_float2(p.k2e, p.k2e));
-            float2 r;
-            asm("{\n.reg .f32 a;\nabs.f32 a, %1;\nex2.approx.ftz.f32 %0, a;\n}\n" : "=f"(r.x) : "f"(y.x));
-            asm("{\n.reg .f32 a;\nabs.f32 a, %1;\nex2.approx.ftz.f32 %0, a;\n}\n" : "=f"(r.y) : "f"(y.y));
-            r = __fadd2_rn(r, make_float2(1.f, 1.f));
-            asm("rcp.approx.ftz.f32 %0, %0;\n" : "+f"(r.x));
-            asm("rcp.approx.ftz.f32 %0, %0;\n" : "+f"(r.y));
-            const float2 t = __ffma2_rn(make_float2(p.m2c, p.m2c), r, make_float2(p.c, p.c));
-            s[j] = pick(x.x, q.x, t.x);
-            s[j + 1] = pick(x.y, q.y, t.y);
-        }
+            for (int j = 0; j < N; j += 2) {
+                const float2 x = make_float2(__uint_as_float(s[j]), __uint_as_float(s[j + 1]));
+                const float2 z = decltype(powers_tag)::value ? x : __fmul2_rn(x, make_float2(p.k, p.k));
+                const float2 q = poly(x, z), y = __fmul2_rn(x, make_float2(p.k2e, p.k2e));
+                float2 r;
+                asm("{\n.reg .f32 a;\nabs.f32 a, %1;\nex2.approx.ftz.f32 %0, a;\n}\n" : "=f"(r.x) : "f"(y.x));
+                asm("{\n.reg .f32 a;\nabs.f32 a, %1;\nex2.approx.ftz.f32 %0, a;\n}\n" : "=f"(r.y) : "f"(y.y));
+                r = __fadd2_rn(r, make_float2(1.f, 1.f));
+                asm("rcp.approx.ftz.f32 %0, %0;\n" : "+f"(r.x));
+                asm("rcp.approx.ftz.f32 %0, %0;\n" : "+f"(r.y));
+                const float2 t = __ffma2_rn(make_float2(p.m2c, p.m2c), r, make_float2(p.c, p.c));
+                s[j] = pick(x.x, q.x, t.x);
+                s[j + 1] = pick(x.y, q.y, t.y);
+            }
+        };
+        if (p.lim_all > 0.f) both(std::true_type{});
+        else both(std::false_type{});
     }
 }
 
@@ -1969,12 +1976,18 @@ int launch_fwd_sm100(const FwdParams& p, cudaStream_t stream) {
     dev.rescale_thr = expm == 1 ? 0.01f * (float)g_rescale_half_x100.load() : kRescaleThreshold;
     dev.soft_cap = p.logits_soft_cap;
     if (p.logits_soft_cap > 0.f) {
-        const float k = p.scale * (1.f / p.logits_soft_cap), k2 = k * k, c0 = dev.scale_log2;
+        const float k = p.scale * (1.f / p.logits_soft_cap), c0 = dev.scale_log2;
         SoftCap& s = dev.cap;
-        // (beyond 1e3 the eighth power of k could overflow)
-        s.lim = fabsf(k) < 1e3f ? 0.5f / fabsf(k) : -1.f;
-        s.c0 = c0; s.c1 = -0.33333069f * (c0 * k2); s.c2 = 0.13324779f * (c0 * k2 * k2);
-        s.c3 = -0.052986056f * (c0 * k2 * k2 * k2); s.c4 = 0.017135002f * (c0 * (k2 * k2) * (k2 * k2));
+        // The coefficients carry powers of k up to the eighth, so that the raw score itself is the variable.  Where the last
+        // one leaves the range in which products keep 24 bits (a scale of 0.0884 with caps above 2000, say), the score is
+        // multiplied by k first instead, in the branch that has both forms.
+        const auto last = [&](float kk) { return 0.017135002f * (c0 * (kk * kk) * (kk * kk)); };
+        const float l = fabsf(last(k * k));
+        const bool powers = fabsf(k) < 1e3f && l > 1e-36f && l < 1e36f;
+        const float kk = powers ? k * k : 1.f;
+        s.lim = 0.5f / fabsf(k); s.lim_all = powers ? s.lim : -1.f; s.k = k;
+        s.c0 = c0; s.c1 = -0.33333069f * (c0 * kk); s.c2 = 0.13324779f * (c0 * kk * kk);
+        s.c3 = -0.052986056f * (c0 * kk * kk * kk); s.c4 = last(kk);
         s.k2e = 2.885390081777927f * k; s.c = copysignf(p.logits_soft_cap * kLog2e, k); s.m2c = -2.f * s.c;
     }
     dev.alibi = (p.bias && p.bias_type == 2) ? (const float*)p.bias : nullptr; dev.alibi_rank = p.bias_rank;

@@ -111,10 +111,11 @@ def test_capped_rows_are_independent(d, add):
 
 
 # One key per sequence and one channel in use: the LSE of a row is its capped score, and the score is exact before the cap.
-# Queries of all sizes from 1e-3 to 4 caps stand side by side in a warp, or each size in warps of its own.
+# Queries of all sizes from 1e-3 to 4 caps stand side by side in a warp, or each size in warps of its own; the caps reach both
+# ends of the range in which the polynomial's coefficients hold powers of scale / cap.
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("scale", [0.0884, 1.0, -0.0884])
-@pytest.mark.parametrize("cap", [0.05, 1.0, 20.0, 900.0])
+@pytest.mark.parametrize("cap", [1e-5, 0.05, 1.0, 20.0, 900.0, 2e3, 1e4, 1e5, 1e6, 1e9])
 @pytest.mark.parametrize("mixed", [False, True])
 def test_capped_score_in_fp32(d, scale, cap, mixed):
     n = 512
