@@ -902,7 +902,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             ctrl->nblk[b] = cost * p.hkv;
             ctrl->items[b] = (uint32_t)nmax;  // (scratch until the work list is written)
         }
-        else ctrl->nblk[b] = min(p.num_levels, (sq + rows_per_block - 1) / rows_per_block);
+        else ctrl->nblk[b] = max(0, min(p.num_levels, (sq + rows_per_block - 1) / rows_per_block));  // (starts that step down: none)
     }
     __syncthreads();
     if (SPLIT) {

@@ -44,3 +44,24 @@ def test_every_row_once(batch, lo, hi, hq, hkv, causal, more):
     o_ref, lse_ref = _reference(q, k, v, nq, nk, causal)
     assert_o_close(o, o_ref)
     assert_lse_close(lse, lse_ref)
+
+
+# Sequence starts whose unused tail holds zeros: the sequence behind the last valid one ends before it begins.  It has no rows,
+# and the others are computed as if it were not there, whichever form the list takes (one item per SM at most; sorted; by level).
+@pytest.mark.parametrize("nq,hq,hkv,d", [([300, 400], 4, 2, 128), ([300, 900, 1], 64, 8, 128), ([700] * 120, 8, 2, 128), ([300, 400], 3, 1, 128),
+                                         ([300, 900, 1], 64, 8, 64)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_starts_with_a_zero_tail(nq, hq, hkv, d, bias):
+    if bias and (d == 64 or sum(nq) > 2000):
+        pytest.skip("(the list of the bias instances: the short ones)")
+    g = torch.Generator(device="cuda").manual_seed(len(nq))
+    q, k, v = (torch.randn((sum(nq), h, d), generator=g, device="cuda").bfloat16() for h in (hq, hkv, hkv))
+    more = {"causal": True, "return_lse": True}
+    if bias:
+        more["bias"] = torch.randn((1, hq, sum(nq), sum(nq)), generator=g, device="cuda").bfloat16()
+    cu = to_seqstarts(nq).cuda()
+    padded = torch.cat([cu, torch.zeros(5, dtype=cu.dtype, device="cuda")])
+    o, lse = ops.fmha_fwd_var_len(q, k, v, padded, padded, max(nq), **more)
+    assert _lib.device_status() == 0
+    o_ref, lse_ref = ops.fmha_fwd_var_len(q, k, v, cu, cu, max(nq), **more)
+    assert torch.equal(o, o_ref) and torch.equal(lse, lse_ref)
