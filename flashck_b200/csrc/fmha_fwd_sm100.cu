@@ -734,7 +734,7 @@ __device__ __forceinline__ void prefill_work_list(Ctrl* ctrl, const Sm100Dev& p)
             const int gi = div_by(w, p.inv_per_group);
             return 0x80000000u | group_item(gi) | ((uint32_t)(w - gi * per_group) << 12);
         };
-        const bool deal = sorted && g <= kDealCtas;
+        const bool deal = sorted && g <= kDealCtas && rounds > 0;  // (0: the list is too long, see above)
         const int last = deal ? rounds - 1 : rounds;
 #pragma unroll 1
         for (int rnd = j; rnd < last; rnd += NTHREADS) ctrl->items[rnd] = item_word(item_of_round(rnd, blockIdx.x, g));

@@ -65,3 +65,20 @@ def test_starts_with_a_zero_tail(nq, hq, hkv, d, bias):
     assert _lib.device_status() == 0
     o_ref, lse_ref = ops.fmha_fwd_var_len(q, k, v, cu, cu, max(nq), **more)
     assert torch.equal(o, o_ref) and torch.equal(lse, lse_ref)
+
+
+# The longest list a CTA can hold (1024 items), sorted and dealt, and one sequence more: that call leaves for the general instance.
+@pytest.mark.parametrize("over", [0, 1])
+def test_longest_list(over):
+    sms, heads = torch.cuda.get_device_properties(0).multi_processor_count, 1023
+    batch = sms * 1024 // heads + over
+    nq = [1 + i % 2 for i in range(batch)]
+    nk = [n + i % 3 for i, n in enumerate(nq)]
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    q, k, v = (torch.randn((sum(n), heads, 128), generator=g, device="cuda").bfloat16() for n in (nq, nk, nk))
+    o, lse = ops.fmha_fwd_var_len(q, k, v, to_seqstarts(nq).cuda(), to_seqstarts(nk).cuda(), max(nq), causal=True, return_lse=True)
+    assert _lib.get_instance_param(0, "last_instance") == 1 - over
+    assert _lib.device_status() == 0
+    o_ref, lse_ref = _reference(q, k, v, nq, nk, True)
+    assert_o_close(o, o_ref)
+    assert_lse_close(lse, lse_ref)
