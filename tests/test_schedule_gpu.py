@@ -1,4 +1,4 @@
-"""The prefill kernel's work list: every query row of every sequence is computed once, whichever way the list is made."""
+"""The hdim-128 prefill kernel's work list: every query row of every sequence is computed once, whichever way the list is made."""
 import pytest
 import torch
 
@@ -9,14 +9,18 @@ from tests.helpers import assert_lse_close, assert_o_close
 pytestmark = pytest.mark.gpu
 
 
-def _reference(q, k, v, nq, nk, causal):
+def _reference(q, k, v, nq, nk, causal, window=-1, bias=None):
     o, lse, group = torch.empty(q.shape, device=q.device), torch.empty((q.shape[1], q.shape[0]), device=q.device), q.shape[1] // k.shape[1]
     a = c = 0
     for n, m in zip(nq, nk):
         kk, vv = (t[c:c + m].float().repeat_interleave(group, 1) for t in (k, v))
         x = torch.einsum("qhd,khd->hqk", q[a:a + n].float(), kk) * q.shape[2] ** -0.5
+        if bias is not None:  # over the packed totals
+            x += bias[0, :, a:a + n, c:c + m].float()
         if causal:
             x.masked_fill_(torch.arange(m, device=q.device) > torch.arange(n, device=q.device)[:, None] + (m - n), float("-inf"))
+        if window >= 0:
+            x.masked_fill_(torch.arange(m, device=q.device) < torch.arange(n, device=q.device)[:, None] + (m - n - window), float("-inf"))
         lse[:, a:a + n] = torch.logsumexp(x, -1)
         o[a:a + n] = torch.einsum("hqk,khd->qhd", torch.softmax(x, -1), vv)
         a, c = a + n, c + m
@@ -65,6 +69,41 @@ def test_starts_with_a_zero_tail(nq, hq, hkv, d, bias):
     assert _lib.device_status() == 0
     o_ref, lse_ref = ops.fmha_fwd_var_len(q, k, v, cu, cu, max(nq), **more)
     assert torch.equal(o, o_ref) and torch.equal(lse, lse_ref)
+
+
+# Equal lengths, whose order is known in closed form: several rounds of items, batches above 2, paired and unpaired heads, even
+# and odd numbers of row tiles (unpaired and odd: a last block of one tile), with the orders by block (mask or bias) and by
+# sequence (neither).
+@pytest.mark.parametrize("batch,n,hq,hkv", [(5, 700, 32, 8), (5, 600, 24, 8), (7, 900, 24, 8), (3, 1200, 32, 32), (4, 1100, 40, 8),
+                                            (21, 129, 16, 2), (160, 100, 3, 1)])
+@pytest.mark.parametrize("causal,window", [(False, -1), (True, -1), (True, 200)])
+@pytest.mark.parametrize("bias", [None, 0, 1])
+def test_equal_lengths(batch, n, hq, hkv, causal, window, bias):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q, k, v = (torch.randn((batch, n, h, 128), generator=g, device="cuda").bfloat16() for h in (hq, hkv, hkv))
+    b = torch.randn((1, hq if bias else 1, n, n), generator=g, device="cuda").bfloat16() if bias is not None else None
+    o, lse = ops.fmha_fwd(q, k, v, causal=causal, window_size=(window, 0) if window >= 0 else (-1, -1), bias=b, return_lse=True)
+    assert _lib.device_status() == 0 and _lib.get_instance_param(0, "last_instance") == 1
+    for i in range(batch):
+        o_ref, lse_ref = _reference(q[i], k[i], v[i], [n], [n], causal, window, b)
+        assert_o_close(o[i], o_ref)
+        assert_lse_close(lse[i], lse_ref)
+
+
+# a bias over packed sequences with more items than SMs (the list of the bias instances by level)
+@pytest.mark.parametrize("hq,hkv", [(32, 8), (40, 8)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_packed_bias_over_several_rounds(hq, hkv, causal):
+    nq = [300, 650, 1, 411]
+    g = torch.Generator(device="cuda").manual_seed(hq)
+    q, k, v = (torch.randn((sum(nq), h, 128), generator=g, device="cuda").bfloat16() for h in (hq, hkv, hkv))
+    b = torch.randn((1, hq, sum(nq), sum(nq)), generator=g, device="cuda").bfloat16()
+    cu = to_seqstarts(nq).cuda()
+    o, lse = ops.fmha_fwd_var_len(q, k, v, cu, cu, max(nq), causal=causal, bias=b, return_lse=True)
+    assert _lib.device_status() == 0 and _lib.get_instance_param(0, "last_instance") == 1
+    o_ref, lse_ref = _reference(q, k, v, nq, nq, causal, bias=b)
+    assert_o_close(o, o_ref)
+    assert_lse_close(lse, lse_ref)
 
 
 # The longest list a CTA can hold (1024 items), sorted and dealt, and one sequence more: that call leaves for the general instance.
