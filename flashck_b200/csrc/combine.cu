@@ -3,8 +3,9 @@
 // (attention_kernels/fmha_fwd_split_kv_combine/fmha_fwd_split_kv_combine_jinja.h:125-140): lse_acc
 // [bs,hq,S,rows], o_acc [bs,hq,S,rows,dv].  The strided form also reads partials gathered from several GPUs
 // ([rank][...] layouts) and can leave the result in fp32, which is what a rank contributes to such a gather.
-// o_acc is read once and is a few MB at most, so what bounds the kernel is its chain of memory round trips: one warp per
-// (batch, head, row) when a row has few splits, several warps per row otherwise (see combine_wide_kernel).
+// The partials in use are read once: from half a megabyte (one token of 32 heads, 32 splits) to some 10-30 MB (9888 rows of
+// dv 128 with 2-6 splits), mostly out of L2.  What bounds the kernel is its chain of memory round trips: one warp per (batch,
+// head, row) when a row has few splits, several warps per row otherwise (see combine_wide_kernel).
 #include "kernels.h"
 
 namespace fck {
@@ -124,7 +125,8 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineDev p) {
 // Several warps per row (one CTA = one row), for rows with many splits: a warp that walks 94 splits four rows at a time
 // pays a memory round trip for every four.  Warp w takes splits w, w + W, ...; it requests its first kAhead rows before
 // it has seen any LSE (a split without keys may hold anything: its row is dropped by its weight of zero, not multiplied),
-// so that a row of W * kAhead splits costs two round trips -- LSE and partials together, then nothing but shared memory.
+// so that a row of up to W * kAhead splits costs one round trip for LSE and partials together, and a longer one another for
+// every further W * kAhead.  All slots of a row are read, those of empty splits too.
 // Merging one token of 32 heads over 128 split slots, 94 in use: 16.4 us with one warp per row, 3.3 us with 16 (back to
 // back in a graph; 24.5 us alone behind its split kernel before).
 template <typename T, int W>
@@ -226,6 +228,7 @@ cudaError_t launch_t(const CombineDev& d, cudaStream_t stream) {
     // warps than that only queue, and the other rows hide a row's round trips.  Measured (us with 1 / 4 / 8 / 16 warps,
     // dv 128): 32 rows x 128 slots 16.4 / 4.9 / 3.7 / 3.3; 256 x 75 9.6 / 4.1 / 3.7 / 4.4; 512 x 20 4.2 / 3.1 / 3.6 /
     // 6.0; 2048 x 16 4.4 / 5.5 / 9.5 / 18; 2048 x 6 3.6 / 5.4 / 9.1 / 17.
+    // (The order of a row's fp32 sum follows from W, and so from the number of rows in the call.)
     const int64_t warps_ok = (int64_t)sm_count() * 16 / (d.items > 0 ? d.items : 1);
     const dim3 g((unsigned)d.items);
     const size_t row = d.dv * sizeof(float);

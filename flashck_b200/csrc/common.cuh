@@ -157,8 +157,8 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // tanh(y) = sign(y) (1 - e^{-2|y|}) / (1 + e^{-2|y|}) on the exp2 and reciprocal units, inline (the library tanhf is a
-// call with a slow path, and a call inside the 128-element score loop costs the loop its scheduling even when the
-// branch around it is not taken).  Relative error below 1e-4 near 0, 1e-6 elsewhere: far inside the rounding of P.
+// call with a slow path).  Relative error up to 1.5e-4 near 0 (1e-7 absolute), 1e-6 from 0.5 on: for the soft cap of the
+// general instance; the tcgen05 instances have a form of their own that keeps its digits near 0.
 constexpr float kLog2e = 1.4426950408889634f;
 __device__ __forceinline__ float tanh_inline(float y) {
     float e;

@@ -438,7 +438,9 @@ struct Ctrl {
     uint32_t tmem_base;
     int abort_flag;
     int num_levels;                     // row-block indices 0 .. num_levels-1
-    int level_start[kMaxLevels + 1];    // first work item of each level; level 0 = highest block index
+    // by level: first work item of each level, level 0 = highest block index; lists of prefill_work_list for lengths of their
+    // own: first group of each sequence; split modes: first unit of each sequence
+    int level_start[kMaxLevels + 1];
     int nblk[kMaxBatch];                // row blocks of each sequence
     int seq_q0[kMaxBatch], seq_sq[kMaxBatch], seq_k0[kMaxBatch], seq_sk[kMaxBatch];  // first row / length, Q and K
     // (prefill: the words behind kMaxRounds hold the sorted groups and the CTAs' loads while the list is made)
@@ -457,9 +459,6 @@ __device__ __forceinline__ int item_of_round(int rnd, int cta, int g) {
     return rnd * g + ((rnd & 1) ? (g - 1 - cta) : cta);
 }
 
-// Work items are ordered by decreasing row-block index (under a causal mask: decreasing cost), then by sequence,
-// then by head, so that the q heads of a GQA group -- which read the same K/V -- run at the same time on
-// neighbouring SMs and share those tiles through L2.  Warp-collective.
 static_assert(1024 + (2 + 2 * KV_SLOTS) * TILE_BYTES + 8 * STAGE_BYTES + sizeof(Ctrl) <= 227 * 1024,
               "tiles, staging buffers and the control block must fit the 227 KB a CTA can have");
 
@@ -513,6 +512,10 @@ __device__ __forceinline__ void expand_item_split(const Ctrl* ctrl, const Sm100D
     it.N = it.nt[0];
 }
 
+// Item `w` of the order by levels (hdim 64, and the lists of prefill_work_list that are neither uniform nor sorted):
+// decreasing row-block index (under a causal mask: decreasing cost), then by sequence, then by head.  Warp-collective.
+// In every order the heads come last, so that the q heads of a GQA group -- which read the same K/V -- run at the same
+// time on neighbouring SMs and share those tiles through L2.
 __device__ __forceinline__ uint32_t find_item(const Ctrl* ctrl, const Sm100Dev& p, int w, int lane) {
     int lo = 0, hi = ctrl->num_levels;  // last level whose start is <= w
     while (hi - lo > 1) {
@@ -969,7 +972,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         }
     }
     // The hdim-64 instances keep their items in order of levels, worked out in place: ptxas' allocation in their role loops
-    // moves with the code in front of them, and with the lists above, inline or called, it came out 2-10 % slower (4 x 4096
+    // moves with the code in front of them, and with the lists above, inline or called, it came out 2-12 % slower (4 x 4096
     // tokens, 32 heads, causal: 386 us; called 412, inline 432).
     constexpr bool LEVELS = SPLIT == 0 && HDIM == 64;
     if constexpr (SPLIT == 0 && !LEVELS) {

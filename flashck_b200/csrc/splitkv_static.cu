@@ -12,7 +12,7 @@
 //     FLASHCK_ERR_UNSUPPORTED and a message that states the size asked for;
 //   * every call on a device uses the same array, which keeps whatever the previous call left there.  Nothing
 //     in it needs to start at zero: the split kernel writes -inf into the LSE slot of every split it does not
-//     fill, and the combine never reads the O slot of such a split.  Two calls that overlap on the GPU (different
+//     fill, and the combine uses nothing of the O slot of such a split.  Two calls that overlap on the GPU (different
 //     streams, or different host threads) race on the array -- serialise them;
 //   * the first call on each device resolves the array's device address (a host-side lookup, no allocation).
 //     Make that first call outside any stream capture.

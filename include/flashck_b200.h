@@ -94,7 +94,8 @@ FLASHCK_API int FmhaFwd(void* q_buf_ptr, void* k_buf_ptr, void* v_buf_ptr, void*
  * sequence's block starts at its first packed row and key); contiguous K/V of the stated lengths only.
  * bias_enum 2 (alibi): bias_buf_ptr holds fp32 slopes, bias_rank_info 0 = [1,hq], 1 = [b,hq]; the score of query i
  * and key j gets -slope * |i + sk - sq - j| added.  logits_soft_cap > 0: score = cap * tanh(score / cap), applied to
- * the scaled score before the bias.  These calls run on the general (mma.sync) instance.
+ * the scaled score before the bias.  On contiguous K/V the tcgen05 instances serve alibi and the soft cap at head dims
+ * 64 and 128 and an elementwise bias at 128; what they do not take runs on the general (mma.sync) instance.
  */
 FLASHCK_API int FmhaFwdBias(void* q_buf_ptr, void* k_buf_ptr, void* v_buf_ptr, void* bias_buf_ptr, void* o_buf_ptr,
             int64_t* q_seq_start_ptr, int64_t* k_seq_start_ptr, int64_t* k_seq_len_ptr, int64_t batch,
