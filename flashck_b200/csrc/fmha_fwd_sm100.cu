@@ -197,6 +197,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -402,6 +410,21 @@ __device__ __forceinline__ void add_f16x2_to(float2& acc, uint32_t v) {
     asm("{\n.reg .f16 l, h;\nmov.b32 {l, h}, %2;\nadd.f32.f16 %0, l, %0;\nadd.f32.f16 %1, h, %1;\n}\n"
         : "+f"(acc.x), "+f"(acc.y)
         : "r"(v));
+}
+
+// O *= alpha for the rows of a warp (one accumulator row per thread, HD columns from `tO`).  Out of line: it runs once or twice
+// per row, and in place the softmax loop jumps over its instructions in every step.
+template <int HD>
+__device__ __noinline__ void rescale_rows(uint32_t tO, float alpha) {
+#pragma unroll 1
+    for (int c = 0; c < HD; c += 16) {
+        uint32_t t[16];
+        tmem_ld16(tO + c, t);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) t[j] = __float_as_uint(__uint_as_float(t[j]) * alpha);
+        tmem_st16(tO + c, t);
+    }
 }
 
 constexpr int kMaxBatch = 256;    // sequences the on-chip schedule can hold (larger batches use the general instance)
@@ -1467,7 +1490,8 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 else off += (p.bias_el_rank == 2 ? (int64_t)it.b * p.hq * plane : 0) + (int64_t)row * p.bias_sk;
                 if (row_ok) bias_row = reinterpret_cast<const unsigned short*>(p.bias_el) + off;
             }
-            for (int n = 0; n < Ni; ++n) {
+            auto step = [&](int n, auto mask_tag) -> bool {
+                constexpr bool MASK = decltype(mask_tag)::value;  // some score of the tile is hidden
                 // warp-uniform outcome: the loads, votes and stores below are warp-collective
                 // The split modes have one Q tile and use the other tile's S columns as a second S buffer: the QK^T of
                 // step n+1 is issued before the PV of step n, so the next S is there when P has been handed over.
@@ -1492,7 +1516,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 }
                 ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctrl->s_full[sb], (SPLIT ? (gstep >> 1) : gstep) & 1u, abort_flag,
                                                                p.status, 0x100 << i));
-                if (!ok) break;
+                if (!ok) return false;
                 tc_fence_after();
                 constexpr int NC = SPLIT == 2 ? 64 : 128;  // columns of the row this thread handles
                 uint32_t sreg[NC];
@@ -1543,14 +1567,18 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         else add_slope(std::false_type{});
                     }
                 }
-                // mask the diagonal and tail tiles
-                const bool need_mask = (key0 + NC > sk) ||
-                                       (p.causal && wr >= 0 && key0 + NC - 1 > tile_first_row + shift + wr) ||
-                                       (WINDOW && p.causal && wl >= 0 && key0 < tile_first_row + BM - 1 + shift - wl);
-                if (need_mask) {
+                // Mask: a warp's 32 rows see a prefix (or, with a left window, a band) of the columns, so most 32-column groups
+                // are seen by all of them or by none.
+                if constexpr (MASK) {
+                    const int hi = row_ok ? limit - key0 : -1, lo = WINDOW ? first_key - key0 : 0;
 #pragma unroll
-                    for (int j = 0; j < NC; ++j)
-                        if (key0 + j > limit || (WINDOW && key0 + j < first_key)) sreg[j] = 0xff800000u;  // -inf
+                    for (int c = 0; c < NC / 32; ++c) {
+                        if (__any_sync(0xffffffffu, c * 32 + 31 > hi || (WINDOW && c * 32 < lo))) {
+#pragma unroll
+                            for (int j = c * 32; j < c * 32 + 32; ++j)
+                                if (j > hi || (WINDOW && j < lo)) sreg[j] = 0xff800000u;  // -inf
+                        }
+                    }
                 }
                 float mx;
                 {
@@ -1574,19 +1602,23 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         // of it.
                         ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctrl->pv_done[sb ^ 1], ((gstep - 1u) >> 1) & 1u,
                                                                        abort_flag, p.status, 0x1000));
-                        if (!ok) break;
+                        if (!ok) return false;
                         tc_fence_after();
                     }
                     const float alpha = grow ? fast_exp2(m_used - mx) : 1.f;  // exp2(-inf) = 0
                     l *= alpha;
+                    if constexpr (F8) {  // (P's range is short: rows grow often)
 #pragma unroll
-                    for (int c = 0; c < HD / 32; ++c) {
-                        uint32_t t[32];
-                        tmem_ld32(tO + c * 32, t);
-                        tmem_wait_ld();
+                        for (int c = 0; c < HD / 32; ++c) {
+                            uint32_t t[32];
+                            tmem_ld32(tO + c * 32, t);
+                            tmem_wait_ld();
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) t[j] = __float_as_uint(__uint_as_float(t[j]) * alpha);
-                        tmem_st32(tO + c * 32, t);
+                            for (int j = 0; j < 32; ++j) t[j] = __float_as_uint(__uint_as_float(t[j]) * alpha);
+                            tmem_st32(tO + c * 32, t);
+                        }
+                    } else {
+                        rescale_rows<HD>(tO, alpha);
                     }
                     tmem_wait_st();
                 }
@@ -1596,10 +1628,9 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 float2 psa = make_float2(0.f, 0.f), psb = make_float2(0.f, 0.f);
                 // P = 2^(S * scale - max) for the 128 columns of the row, 64 at a time.  NPOLY8 of every 8 column
                 // pairs take the polynomial; tiles with masked (-inf) entries use the exp2 unit only, which returns
-                // exact zeros for them.  The two variants are separate straight-line loops so that the scheduler
-                // can interleave exp2-unit and FMA-pipe work across column pairs.
-                auto exp_half = [&](int c, auto use_poly_tag) {
-                    [[maybe_unused]] constexpr int NP = decltype(use_poly_tag)::value;
+                // exact zeros for them.
+                auto exp_half = [&](int c) {
+                    [[maybe_unused]] constexpr int NP = MASK ? 0 : NPOLY8;
                     if constexpr (F8) {
                         // 8-bit P: stretched by scale_p, rounded (saturating) to the operand format, four keys per
                         // TMEM column; the row sum takes the unrounded values
@@ -1619,30 +1650,30 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         }
                         tmem_st16(tSb + c * 16, pk8);
                     } else {
-                    uint32_t pk[32];
+                        uint32_t pk[32];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const int e = c * 64 + 2 * j;
-                        const float2 x = __ffma2_rn(make_float2(__uint_as_float(sreg[e]), __uint_as_float(sreg[e + 1])), sc2, nm2);
-                        if constexpr (HEXP) {
-                            const uint32_t ph = ex2_f16x2(pack_f16x2(x.x, x.y));
-                            if constexpr (std::is_same<T, __half>::value) {  // P is the unit's result as it stands
-                                if (j & 1) add_f16x2_to(psb, ph); else add_f16x2_to(psa, ph);
-                                pk[j] = ph;
-                            } else {
-                                const float2 pr = unpack_f16x2(ph);
-                                if (j & 1) psb = __fadd2_rn(psb, pr); else psa = __fadd2_rn(psa, pr);
-                                pk[j] = Elem<T>::pack2(pr.x, pr.y);
+                        for (int j = 0; j < 32; ++j) {
+                            const int e = c * 64 + 2 * j;
+                            const float2 x = __ffma2_rn(make_float2(__uint_as_float(sreg[e]), __uint_as_float(sreg[e + 1])), sc2, nm2);
+                            if constexpr (HEXP) {
+                                const uint32_t ph = ex2_f16x2(pack_f16x2(x.x, x.y));
+                                if constexpr (std::is_same<T, __half>::value) {  // P is the unit's result as it stands
+                                    if (j & 1) add_f16x2_to(psb, ph); else add_f16x2_to(psa, ph);
+                                    pk[j] = ph;
+                                } else {
+                                    const float2 pr = unpack_f16x2(ph);
+                                    if (j & 1) psb = __fadd2_rn(psb, pr); else psa = __fadd2_rn(psa, pr);
+                                    pk[j] = Elem<T>::pack2(pr.x, pr.y);
+                                }
+                                continue;
                             }
-                            continue;
+                            float2 pr;
+                            if (NP > 0 && ((j * NP) & 7) < NP) pr = exp2_poly2(x);
+                            else { pr.x = ex2_fast(x.x); pr.y = ex2_fast(x.y); }
+                            if (j & 1) psb = __fadd2_rn(psb, pr); else psa = __fadd2_rn(psa, pr);
+                            pk[j] = Elem<T>::pack2(pr.x, pr.y);
                         }
-                        float2 pr;
-                        if (NP > 0 && ((j * NP) & 7) < NP) pr = exp2_poly2(x);
-                        else { pr.x = ex2_fast(x.x); pr.y = ex2_fast(x.y); }
-                        if (j & 1) psb = __fadd2_rn(psb, pr); else psa = __fadd2_rn(psa, pr);
-                        pk[j] = Elem<T>::pack2(pr.x, pr.y);
-                    }
-                    tmem_st32(tSb + (SPLIT == 2 ? khalf : c) * 32, pk);
+                        tmem_st32(tSb + (SPLIT == 2 ? khalf : c) * 32, pk);
                     }
                 };
                 // Prefill forms: P is handed over in two halves (a barrier each: with one barrier the second arrival could
@@ -1656,15 +1687,9 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                         if (lane == 0) mbar_arrive(&ctrl->p_full[sb]);
                     }
                 };
-                if (need_mask) {
-                    exp_half(0, std::integral_constant<int, 0>{});
-                    hand_over_first_half();
-                    if (SPLIT != 2) exp_half(1, std::integral_constant<int, 0>{});
-                } else {
-                    exp_half(0, std::integral_constant<int, NPOLY8>{});
-                    hand_over_first_half();
-                    if (SPLIT != 2) exp_half(1, std::integral_constant<int, NPOLY8>{});
-                }
+                exp_half(0);
+                hand_over_first_half();
+                if (SPLIT != 2) exp_half(1);
                 if (SPLIT == 2) {  // this copy of the row gives the other 64 keys no weight
                     uint32_t zero[32];
 #pragma unroll
@@ -1676,6 +1701,19 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(HALVES ? &ctrl->p_full2[sb] : &ctrl->p_full[sb]);
+                return true;
+            };
+            for (int n = 0; ok && n < Ni; ++n) {
+                // The diagonal and tail tiles take a copy of the step of their own, so that the others' code is one straight run:
+                // a jump over the 256 instructions of the mask, or over the rescale of O, costs 100-200 clocks of a step's 3250
+                // (now 2950).  us before / after: 16 x 512-4096 tokens causal 998 / 945; hdim 64, 32 x 1025 tokens 313 / 300;
+                // window with a cap 249 / 240; 2 x 2048 with a bias per head 216 / 204; 8-bit operands 918 / 910.
+                constexpr int NCM = SPLIT == 2 ? 64 : 128;
+                const int key0 = (it.n0 + n) * BN + khalf * 64;
+                const bool need_mask = (key0 + NCM > sk) ||
+                                       (p.causal && wr >= 0 && key0 + NCM - 1 > tile_first_row + shift + wr) ||
+                                       (WINDOW && p.causal && wl >= 0 && key0 < tile_first_row + BM - 1 + shift - wl);
+                ok = need_mask ? step(n, std::true_type{}) : step(n, std::false_type{});
             }
             if (!ok) break;
             sc += Ni;
