@@ -70,17 +70,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_pybind(force: bool = False) -> str:
-    """Compiles ``csrc/pybind/flash_ck.cpp`` -- the pybind11 / PyTorch binding over the C++ operator API -- into
+    """Compiles ``csrc/pybind/*.cpp`` -- the pybind11 / PyTorch binding over the C++ operator API, and the calls of ``ops`` -- into
     ``flashck_b200/flash_ck<ext suffix>`` with g++, linked against ``libflashck_b200.so`` (found at run time next to the
     module) and the torch libraries of this interpreter."""
     import sysconfig
 
     import torch
     from torch.utils import cpp_extension as ce
-    src = os.path.join(CSRC, "pybind", "flash_ck.cpp")
+    srcs = [os.path.join(CSRC, "pybind", f) for f in ("flash_ck.cpp", "calls.cpp")]
     out = os.path.join(HERE, "flash_ck" + sysconfig.get_config_var("EXT_SUFFIX"))
     lib = build()
-    deps = [src, lib, os.path.join(HERE, "..", "include", "flashck", "fmha", "fmha_fwd.h"),
+    deps = [*srcs, lib, os.path.join(HERE, "..", "include", "flashck", "fmha", "fmha_fwd.h"),
             os.path.join(HERE, "..", "include", "flashck_b200.h")]
     if not force and os.path.exists(out) and os.path.getmtime(out) >= _newest(deps):
         return out
@@ -95,11 +95,11 @@ def build_pybind(force: bool = False) -> str:
     for inc in ce.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda_home, "include"),
                                      os.path.join(HERE, "..", "include")]:
         cmd += ["-isystem" if "torch" in inc or "cuda" in inc else "-I", inc]
-    cmd += [src, "-o", out, "-L", torch_lib, "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python",
+    cmd += [*srcs, "-o", out, "-L", torch_lib, "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python",
             "-L", HERE, "-l:libflashck_b200.so", f"-Wl,-rpath,{torch_lib}", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
-        raise RuntimeError(f"g++ failed for {src}:\n{r.stdout}\n{r.stderr[-6000:]}")
+        raise RuntimeError(f"g++ failed for {srcs}:\n{r.stdout}\n{r.stderr[-6000:]}")
     return out
 
 

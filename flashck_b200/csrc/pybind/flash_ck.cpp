@@ -285,7 +285,12 @@ at::Tensor fmha_fwd_appendkv(at::Tensor q, at::Tensor k_cache, at::Tensor v_cach
 
 }  // namespace pytorch
 
+namespace calls {
+void add_calls(PyObject* module);  // calls.cpp
+}
+
 PYBIND11_MODULE(flash_ck, m) {
+    calls::add_calls(m.ptr());
     m.doc() = "FlashCK attention path for B200 (PyTorch extension over libflashck_b200.so)";
 
     // enums (core/pybind/pybind_helper.h:3-29 binds DataType; the attention enums follow core/profiling/attention/fmha_library.h)

@@ -20,6 +20,7 @@ from typing import Optional, Sequence, Tuple
 import torch
 
 from .. import _lib
+from ..utils import flags
 from ..utils.enums import MaskEnum, RopeEnum
 
 __all__ = [
@@ -77,6 +78,27 @@ _HERE = contextlib.nullcontext()
 
 def _on(device: torch.device):
     return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+# Plain calls run in the compiled binding (csrc/pybind/calls.cpp: the same checks, allocations and C call; 2 x 128 tokens 24 us a
+# call in Python, 7.0 there).  It answers None for a call that it cannot check completely; the code below then takes it.
+_NATIVE = None  # the binding, or False where it has not been built
+_TUNING_DIR = flags.flag("FC_TUNING_DB_DIR")  # (set: the call may have to tune first)
+
+
+def _native():
+    """The compiled binding, or False: not built, or tuning is on."""
+    global _NATIVE
+    if _TUNING_DIR.value:
+        return False
+    if _NATIVE is None:
+        _lib.lib()
+        try:
+            from .. import flash_ck
+            _NATIVE = flash_ck
+        except ImportError:
+            _NATIVE = False
+    return _NATIVE
 
 
 def _mask(causal: bool, window_size: Sequence[int], mask_type: Optional[int]) -> Tuple[int, int, int]:
@@ -180,6 +202,11 @@ def fmha_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: Option
     (and LSE ``[b, hq, sq]`` when ``return_lse``).  ``bias`` ``[1|b, 1|hq, sq, sk]`` (q's dtype) is added to the scaled
     scores; ``alibi_slopes`` fp32 ``[1|b, hq]`` adds ``-slope * |i + sk - sq - j|``; ``logits_soft_cap`` > 0 caps the
     scaled scores with ``cap * tanh(score / cap)`` first."""
+    native = _native()
+    if native and bias is None and alibi_slopes is None:
+        r = native._call_forward(q, k, v, None, None, 0, scale, causal, window_size, mask_type, return_lse, logits_soft_cap)
+        if r is not None:
+            return r if r.__class__ is not int else _lib.check(r, "FmhaFwd")
     for n, t in (("q", q), ("k", k), ("v", v)):
         _check_cuda(n, t, getattr(q, "dtype", None))
         if t.dim() != 4:
@@ -277,6 +304,12 @@ def fmha_fwd_var_len(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqle
     Returns o ``[total_q, hq, dv]`` (and LSE ``[hq, total_q]``).  ``bias`` is ``[1, 1|hq, total_q, total_k]`` here (the
     reference's group-mode shape: one plane over the packed rows and keys, of which every sequence uses its own block);
     ``alibi_slopes`` and ``logits_soft_cap`` as in :func:`fmha_fwd`."""
+    native = _native()
+    if native and bias is None and alibi_slopes is None and cu_seqlens_q is not None:
+        r = native._call_forward(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, scale, causal, window_size, mask_type,
+                                 return_lse, logits_soft_cap)
+        if r is not None:
+            return r if r.__class__ is not int else _lib.check(r, "FmhaFwd")
     for n, t in (("q", q), ("k", k), ("v", v)):
         _check_cuda(n, t, getattr(q, "dtype", None))
         if t.dim() != 3:
@@ -360,6 +393,12 @@ def fmha_fwd_paged_kv_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
 
     q ``[b, sq, hq, d]`` or packed ``[total_q, hq, d]`` with ``cu_seqlens_q``; pools ``[pages, page, hkv, *]``;
     ``block_table`` int32 ``[b, pages_per_seq]``; ``seqlen_k`` int32 ``[b]``."""
+    native = _native()
+    if native and cache_batch_idx is None and alibi_slopes is None:
+        r = native._call_paged_prefill(q, k_pool, v_pool, block_table, seqlen_k, cu_seqlens_q, max_seqlen_q, scale, causal,
+                                       window_size, mask_type, return_lse)
+        if r is not None:
+            return r if r.__class__ is not int else _lib.check(r, "FmhaFwdPagedKVPrefill")
     _check_cuda("q", q)
     _check_cuda("k_pool", k_pool, q.dtype)
     _check_cuda("v_pool", v_pool, q.dtype)
@@ -510,6 +549,12 @@ def fmha_fwd_splitkv(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     ``seqlen_k`` int32 ``[b]``.  Contiguous: ``[b_cache, sk, hkv, *]`` (+ optional ``seqlen_k``,
     ``cache_batch_idx``) or packed ``[total_k, hkv, *]`` with ``cu_seqlens_k``.
     ``combine=False`` returns the raw ``(lse_acc, o_acc)`` workspaces."""
+    native = _native()
+    if native and cache_batch_idx is None and cu_seqlens_k is None and workspace is None and combine and alibi_slopes is None:
+        r = native._call_splitkv(q, k_cache, v_cache, seqlen_k, block_table, cu_seqlens_q, max_seqlen_q, num_splits, scale,
+                                 causal, window_size, mask_type, return_lse)
+        if r is not None:
+            return r if r.__class__ is not int else _lib.check(abs(r), "FmhaFwdSplitKV" if r > 0 else "FmhaFwdSplitKVCombine")
     _check_cuda("q", q)
     _check_cuda("k_cache", k_cache, q.dtype)
     _check_cuda("v_cache", v_cache, q.dtype)
@@ -588,6 +633,13 @@ def fmha_fwd_append_kv(q: Optional[torch.Tensor], k_cache: torch.Tensor, v_cache
     Batch mode: q ``[b, sq, hq, d]``, knew ``[b, n, hkv, d]``, vnew ``[b, n, hkv, dv]``.  Varlen: packed
     tensors with ``cu_seqlens_q`` / ``cu_seqlens_knew`` (int64 ``[b+1]``).  Returns ``q`` (rotated)."""
     rope = int(rope)
+    native = _native()
+    if native and cache_batch_idx is None:
+        r = native._call_append_kv(q, k_cache, v_cache, knew, vnew, seqlen_k, rotary_cos, rotary_sin, rope, rotary_dim,
+                                   block_table, cu_seqlens_q, cu_seqlens_knew)
+        if r is not None:
+            _lib.check(r, "FmhaFwdAppendKV")
+            return q
     if rope != RopeEnum.NONE and (rotary_cos is None or rotary_sin is None):
         raise ValueError("rotary_cos / rotary_sin are required unless rope == RopeEnum.NONE")
     _check_cuda("k_cache", k_cache)

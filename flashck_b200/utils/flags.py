@@ -83,6 +83,11 @@ def _lookup(name: str) -> _Flag:
     return flag
 
 
+def flag(name: str) -> _Flag:
+    """The flag itself; its ``value`` follows later settings."""
+    return _FLAGS[name]
+
+
 def get_flag(name: str):
     """The flag's value in its own type."""
     return _lookup(name).value
