@@ -59,3 +59,29 @@ def test_growing_maximum(jump, rows, d, left):
     o_ref, lse_ref = _reference(q, k, v, left, 0)
     assert_o_close(o, o_ref)
     assert_lse_close(lse, lse_ref)
+
+
+# 8-bit operands: the steps without a hidden score are a range worked out ahead, and O is rescaled under the exponentials.  P is
+# rounded to 3 (E4M3) or 2 (E5M2) bits behind the leading one: an element of O is off by at most half a unit in the last place of
+# every P, 2^-4 or 2^-3 of the attention over |V|, and by the rounding of O to bf16 (2^-9 of it).
+@pytest.mark.parametrize("dtype,ulp", [(torch.float8_e4m3fn, 2.0 ** -4), (torch.float8_e5m2, 2.0 ** -3)])
+@pytest.mark.parametrize("n,m", [(1, 1), (97, 96), (128, 129), (129, 225), (200, 128), (300, 640)])
+@pytest.mark.parametrize("left,right", [(-1, -1), (-1, 0), (0, 0), (31, 0), (40, 33), (-1, 64), (150, -1), (300, 0)])
+@pytest.mark.parametrize("grow", [False, True])
+def test_eight_bit_steps(dtype, ulp, n, m, left, right, grow):
+    q, k, v = _inputs(n, m, 4, 2, 128, n + m)
+    if grow:  # the maximum rises from tile to tile, for one row of a warp
+        k[..., 0] = torch.arange(m, device="cuda").div(128, rounding_mode="floor")[None, :, None] * 2.0
+        q[..., 0] = 0.0
+        q[:, 5::32, :, 0] = 8.0
+    q8, k8, v8 = (x.to(dtype) for x in (q, k, v))
+    o, lse = ops.fmha_fwd_fp8(q8, k8, v8, scale_p=256.0, scale_o=1 / 256.0, window_size=(left, right), out_dtype=torch.bfloat16,
+                              return_lse=True)
+    assert _lib.get_instance_param(0, "last_instance") == 1
+    qd, kd, vd = (x.float() for x in (q8, k8, v8))
+    o_ref, lse_ref = _reference(qd, kd, vd, left, right)
+    bound = _reference(qd, kd, vd.abs(), left, right)[0] * ulp + o_ref.abs() * 2.0 ** -9
+    # (a P below the smallest normal number keeps fewer bits: 2^-7 / 256 of the largest P and key, E5M2 far less)
+    bound += m * 2.0 ** -10 / 256 * vd.abs().max() + 1e-6
+    assert ((o.float() - o_ref).abs() <= bound).all()
+    assert_lse_close(lse, lse_ref)
