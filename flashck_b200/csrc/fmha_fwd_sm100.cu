@@ -15,6 +15,7 @@ FCK_SM100_HDIM64(FCK_EXTERN, __half) FCK_SM100_HDIM64(FCK_EXTERN, __nv_bfloat16)
 FCK_SM100_EXTRA(FCK_EXTERN, __half) FCK_SM100_EXTRA(FCK_EXTERN, __nv_bfloat16)
 FCK_SM100_EXTRA64(FCK_EXTERN, __half) FCK_SM100_EXTRA64(FCK_EXTERN, __nv_bfloat16)
 FCK_SM100_BIAS(FCK_EXTERN, __half) FCK_SM100_BIAS(FCK_EXTERN, __nv_bfloat16)
+FCK_SM100_TMA_BIAS(FCK_EXTERN, __half) FCK_SM100_TMA_BIAS(FCK_EXTERN, __nv_bfloat16)
 FCK_SM100_FP8(FCK_EXTERN, f8e4m3_t) FCK_SM100_FP8(FCK_EXTERN, f8e5m2_t)
 FCK_SM100_SPLIT(FCK_EXTERN_SPLIT, __half) FCK_SM100_SPLIT(FCK_EXTERN_SPLIT, __nv_bfloat16)
 
@@ -95,6 +96,14 @@ bool fwd_sm100_supported(const FwdParams& p) {
     return true;
 }
 
+// An elementwise bias by TMA: its rows start on 16-byte boundaries (a whole number of 8 keys, an aligned buffer), a row holds at
+// least one box, and a sequence's block starts at a row's first key (batch mode: in the packed form it starts anywhere, and a
+// copy must start on a 16-byte boundary).  Everything else is fetched by the softmax threads.
+static bool bias_by_tma(const FwdParams& p) {
+    return !p.seqstart_q && p.seqlen_k >= 64 && p.seqlen_k % 8 == 0 && (reinterpret_cast<uintptr_t>(p.bias) & 15u) == 0 &&
+           p.seqlen_q < (1ll << 31) && p.seqlen_k < (1ll << 31);
+}
+
 int launch_fwd_sm100(const FwdParams& p, cudaStream_t stream) {
     int* status = device_status_ptr();
     if (!status) return FLASHCK_ERR_CUDA;
@@ -163,6 +172,10 @@ int launch_fwd_sm100(const FwdParams& p, cudaStream_t stream) {
         dev.rescale_thr = kRescaleThreshold;
         dev.bias_el = p.bias; dev.bias_el_rank = p.bias_rank;
         dev.bias_sk = p.seqlen_k; dev.bias_sq = p.seqstart_q ? p.total_q : p.seqlen_q;
+        if (bias_by_tma(p)) {
+            if (window) return bf16 ? launch_t<__nv_bfloat16, 0, 13, 0>(p, dev, stream) : launch_t<__half, 0, 13, 0>(p, dev, stream);
+            return bf16 ? launch_t<__nv_bfloat16, 0, 12, 0>(p, dev, stream) : launch_t<__half, 0, 12, 0>(p, dev, stream);
+        }
         if (window) return bf16 ? launch_t<__nv_bfloat16, 0, 5, 0>(p, dev, stream) : launch_t<__half, 0, 5, 0>(p, dev, stream);
         return bf16 ? launch_t<__nv_bfloat16, 0, 4, 0>(p, dev, stream) : launch_t<__half, 0, 4, 0>(p, dev, stream);
     }

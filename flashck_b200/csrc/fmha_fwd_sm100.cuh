@@ -112,6 +112,11 @@ struct Sm100Dev {
     int64_t bias_sk, bias_sq;
 };
 
+// TMA_BIAS instances: the bias as a tensor map [planes, rows, keys], boxes of 64 keys x 128 rows.
+struct Sm100DevBias : Sm100Dev {
+    CUtensorMap map_bias;
+};
+
 // ---- PTX wrappers ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
     uint64_t d = 0;
@@ -453,6 +458,7 @@ struct Ctrl {
     uint64_t s_full[2], p_full[2], o_full[2];
     uint64_t p_full2[2];  // prefill forms: the second half of P (keys 64-127) has been written (p_full: the first half)
     uint64_t pv_done[2];  // split modes: the PV that read S/P buffer b is complete (buffer b may take the next S)
+    uint64_t b_full[2], b_empty[2];  // TMA_BIAS: the bias tile of Q tile 0 / 1
     uint64_t v_tail;      // paged V: the copies of a tile that holds the end of its sequence (cleaned up before v_full)
     uint32_t tmem_base;
     int abort_flag;
@@ -796,6 +802,12 @@ __device__ __noinline__ void prefill_work_list_call(Ctrl* ctrl, const Sm100Dev& 
 //          columns at a time and adds the bias words as it arrives, so that scores and bias are never live in full
 //          together.  (Fetching through the warp -- four lanes per row, the block handed on through shared memory --
 //          measured the same; fetching a step ahead spilled and lost.)  Implies the score arithmetic of EXTRA.
+// VAR bit 3 (TMA_BIAS, with bit 2): the bias tile of a step (128 rows x 128 keys, 32 KB per Q tile) comes through shared memory, loaded
+//          by the producer a step ahead.  Fetched by the softmax threads, a row each, it bounds the step: 32 lines per load
+//          instruction and an L2 round trip on the chain S -> P, 11800 clocks a step against 2950 without a bias.  The tiles take
+//          the room of the second K and the second V slot: K of step n + 1 has the softmax of step n to arrive, V of step n + 1 that
+//          of step n + 1, and a bias tile is read at the start of its step.  2 x 2048 tokens, 16 heads, a plane per head: 216 -> 109 us.
+//          For whole bias rows of 16-byte pieces (see bias_by_tma).
 // VAR bit 0 (WINDOW): the mask has a left window or a right window other than 0 (everything but no mask / causal); a separate
 // instance, so that the common masks do not carry the second bound of the visible range through the softmax loop.
 // SPLIT 1: the split-KV form described at Sm100Dev (one Q tile per item; work cut as described at kItemCostDefault).  The S
@@ -816,7 +828,7 @@ template <typename T, int EXPM, int VAR, int SPLIT, int HDIM = 128>
 __global__ void __launch_bounds__(NTHREADS, 1)
 fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
-                      const __grid_constant__ Sm100Dev p) {
+                      const __grid_constant__ std::conditional_t<(VAR & 8) != 0, Sm100DevBias, Sm100Dev> p) {
     extern __shared__ uint8_t smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // head dim of this instance (128, or 64 for the prefill forms): the names below shadow the file-scope constants
@@ -830,6 +842,8 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                   "the 8-bit instances: hdim 128, prefill forms, fp32 exponentials, no score additions");
     constexpr bool WINDOW = (VAR & 1) != 0;  // the mask has a second bound (see above)
     constexpr bool BIAS = (VAR & 4) != 0;    // an elementwise bias tensor on the scaled scores
+    constexpr bool TMA_BIAS = (VAR & 8) != 0;
+    static_assert(!TMA_BIAS || (BIAS && HDIM == 128), "a bias through shared memory takes the room of a K and a V slot of hdim 128");
     constexpr bool EXTRA = (VAR & 2) != 0 || BIAS;   // ALiBi and / or a logits soft cap on the scaled scores
     static_assert(!BIAS || (SPLIT == 0 && EXPM == 0 && !F8), "the bias instances are prefill forms with fp32 exponentials");
     constexpr int NPOLY8 = EXPM >= 11 ? EXPM - 10 : 0;
@@ -842,10 +856,12 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     uint8_t* sQ = base;                                  // 2 tiles
     // The split modes have one Q tile; the room of the second one is a third K slot: with a single tile per item
     // the step is short, and two K tiles ahead keep the loads in flight that the HBM rate needs.
-    constexpr int KS = SPLIT ? 3 : 2;
+    constexpr int KS = SPLIT ? 3 : TMA_BIAS ? 1 : 2;
+    constexpr int KV_SLOTS = TMA_BIAS ? 1 : 2;  // (V slots)
     uint8_t* sK = base + (SPLIT ? 1 : 2) * TILE_BYTES;   // KS tiles
     uint8_t* sV = sK + KS * TILE_BYTES;                  // KV_SLOTS tiles
-    uint8_t* sStage = sV + KV_SLOTS * TILE_BYTES;        // 8 x STAGE_BYTES: O chunks of the softmax warps
+    uint8_t* sBias = sV + KV_SLOTS * TILE_BYTES;         // TMA_BIAS: 2 tiles
+    uint8_t* sStage = sBias + (TMA_BIAS ? 2 * TILE_BYTES : 0);  // 8 x STAGE_BYTES: O chunks of the softmax warps
     Ctrl* ctrl = reinterpret_cast<Ctrl*>(sStage + 8 * STAGE_BYTES);
     volatile int* abort_flag = &ctrl->abort_flag;
 
@@ -867,6 +883,8 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
             mbar_init(&ctrl->p_full2[i], 4);
             mbar_init(&ctrl->o_full[i], 1);
             mbar_init(&ctrl->pv_done[i], 1);
+            mbar_init(&ctrl->b_full[i], 1);
+            mbar_init(&ctrl->b_empty[i], 4);
         }
         ctrl->abort_flag = 0;
         ctrl->num_levels = p.num_levels;
@@ -1047,8 +1065,10 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 tma_prefetch_desc(&map_q);
                 tma_prefetch_desc(&map_k);
                 tma_prefetch_desc(&map_v);
+                if constexpr (TMA_BIAS) tma_prefetch_desc(&p.map_bias);
             }
             uint32_t kv_cnt = 0, q_cnt = 0;  // K/V tiles and Q loads issued so far (ring positions)
+            [[maybe_unused]] uint32_t b_cnt[2] = {0, 0};  // TMA_BIAS: bias tiles issued so far
             uint32_t tail_cnt = 0;           // tiles that went through v_tail (its parity)
             // Paged pools are read in chunks of min(page, 128) tokens: one TMA box per chunk and 64-column half.
             // A chunk that the sequence only partly fills is the tail of its last page, and what lies behind the
@@ -1098,6 +1118,20 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                             mbar_expect_tx(&ctrl->k_full[sk_], TILE_BYTES);
                             for (int hb = 0; hb < HB; ++hb)
                                 tma_load_3d(sK + sk_ * TILE_BYTES + hb * HALF_BYTES, &map_k, &ctrl->k_full[sk_], hb * XB, it.kh, row);
+                            if constexpr (TMA_BIAS) {  // (rows and keys behind the ends come as zeros)
+                                for (int i = 0; ok && i < 2; ++i) {
+                                    if (n >= it.nt[i]) continue;
+                                    const int plane = p.bias_el_rank == 0 ? 0 : it.h[i] + (p.bias_el_rank == 2 ? it.b * p.hq : 0);
+                                    ok = mbar_wait_bounded(&ctrl->b_empty[i], (b_cnt[i] & 1u) ^ 1u, abort_flag, p.status, 0x11 + i);
+                                    if (!ok) break;
+                                    ++b_cnt[i];
+                                    mbar_expect_tx(&ctrl->b_full[i], TILE_BYTES);
+                                    for (int hb = 0; hb < 2; ++hb)
+                                        tma_load_3d(sBias + i * TILE_BYTES + hb * HALF_BYTES, &p.map_bias, &ctrl->b_full[i],
+                                                    (it.n0 + n) * BN + hb * 64, it.row0[i], plane);
+                                }
+                                if (!ok) break;
+                            }
                             if (!(ok = mbar_wait_bounded(&ctrl->v_empty[s], ph ^ 1u, abort_flag, p.status, 0x20))) break;
                             mbar_expect_tx(&ctrl->v_full[s], TILE_BYTES);
                             for (int hb = 0; hb < HB; ++hb)
@@ -1320,7 +1354,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                             // probe costs the issuing thread ~100 clocks -- between PV0 and QK0 those would be idle
                             // clocks of the tensor pipe
                             if (!(ok = wait_all(&ctrl->v_full[s], ph, abort_flag, p.status, 0x42))) break;
-                            if (n + 1 < N) {
+                            if (!TMA_BIAS && n + 1 < N) {
                                 if (!(ok = wait_all(&ctrl->k_full[s1], ph1, abort_flag, p.status, 0x44))) break;
                             }
                             if (n < N0) {
@@ -1338,6 +1372,10 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                                 }
                                 if (n == N0 - 1) commit(&ctrl->o_full[0]);
                             } else {
+                                tc_fence_after();
+                            }
+                            if (TMA_BIAS && n + 1 < N) {  // (with one slot K of the next step may still be on its way)
+                                if (!(ok = wait_all(&ctrl->k_full[s1], ph1, abort_flag, p.status, 0x44))) break;
                                 tc_fence_after();
                             }
                             if (n + 1 < N0) { issue_qk(0, s1); commit(&ctrl->s_full[0]); }
@@ -1495,8 +1533,8 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 const uint32_t tSb = SPLIT ? lane_addr + sb * 128 : tS;
                 const int key0 = (it.n0 + n) * BN + khalf * 64;
                 [[maybe_unused]] const bool capped = EXTRA && p.soft_cap > 0.f;
-                [[maybe_unused]] uint4 bw[BIAS ? 16 : 1];  // the 128 bias values of this thread's row and key tile
-                if constexpr (BIAS) {  // (issued before the wait for S)
+                [[maybe_unused]] uint4 bw[BIAS && !TMA_BIAS ? 16 : 1];  // the 128 bias values of this thread's row and key tile
+                if constexpr (BIAS && !TMA_BIAS) {  // (issued before the wait for S)
 #pragma unroll
                     for (int v = 0; v < 16; ++v) bw[v] = load_bias_piece(bias_row, key0 + v * 8, sk - key0 - v * 8);
                     // The next tile's values on their way to L2: no register holds them, and the loads then wait for L2 only
@@ -1516,16 +1554,27 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 tc_fence_after();
                 constexpr int NC = SPLIT == 2 ? 64 : 128;  // columns of the row this thread handles
                 uint32_t sreg[NC];
+                if constexpr (TMA_BIAS) {
+                    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&ctrl->b_full[i], gstep & 1u, abort_flag, p.status, 0x4000 << i));
+                    if (!ok) return false;
+                }
                 if constexpr (BIAS) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         tmem_ld32(tSb + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&sreg[c * 32]));
+                        [[maybe_unused]] uint4 bs[TMA_BIAS ? 4 : 1];  // 32 keys of the row: 16-byte pieces in the 128-byte swizzle
+                        if constexpr (TMA_BIAS) {
+#pragma unroll
+                            for (int v = 0; v < 4; ++v)
+                                bs[v] = *reinterpret_cast<const uint4*>(sBias + i * TILE_BYTES + (c >> 1) * HALF_BYTES + r * 128 +
+                                                                        ((((c & 1) * 4 + v) ^ (r & 7)) << 4));
+                        }
                         tmem_wait_ld();
                         if (capped) soft_cap_scores<32>(&sreg[c * 32], p.cap);
                         const float mul = capped ? 1.f : p.scale_log2;  // (the two products of the sum in base-2 units)
 #pragma unroll
                         for (int j = 0; j < 32; j += 2) {
-                            const uint4 q4 = bw[c * 4 + (j >> 3)];
+                            const uint4 q4 = TMA_BIAS ? bs[TMA_BIAS ? j >> 3 : 0] : bw[TMA_BIAS ? 0 : c * 4 + (j >> 3)];
                             const uint32_t w = ((j >> 1) & 3) == 0 ? q4.x : ((j >> 1) & 3) == 1 ? q4.y : ((j >> 1) & 3) == 2 ? q4.z : q4.w;
                             const float2 b2 = __fmul2_rn(bias_pair<T>(w), make_float2(kLog2e, kLog2e));
                             const float2 x = __ffma2_rn(make_float2(__uint_as_float(sreg[c * 32 + j]), __uint_as_float(sreg[c * 32 + j + 1])),
@@ -1533,6 +1582,10 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                             sreg[c * 32 + j] = __float_as_uint(x.x);
                             sreg[c * 32 + j + 1] = __float_as_uint(x.y);
                         }
+                    }
+                    if constexpr (TMA_BIAS) {  // the next step's tile may come
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&ctrl->b_empty[i]);
                     }
                 } else {
 #pragma unroll
@@ -1936,6 +1989,23 @@ inline int make_map_o(CUtensorMap* map, const void* base, int dtype, int64_t row
     return FLASHCK_OK;
 }
 
+// An elementwise bias [planes, rows, keys] as boxes of 64 keys x 128 rows (128-byte rows, 128-byte swizzle).
+inline int make_map_bias(CUtensorMap* map, const void* base, int dtype, int64_t planes, int64_t rows, int64_t keys) {
+    PFN_encodeTiled enc = get_encode_tiled();
+    FCK_REQUIRE(enc != nullptr, FLASHCK_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    const cuuint64_t dims[3] = {(cuuint64_t)keys, (cuuint64_t)rows, (cuuint64_t)planes};
+    const cuuint64_t strides[2] = {(cuuint64_t)(keys * 2), (cuuint64_t)(rows * keys * 2)};
+    const cuuint32_t box[3] = {64, (cuuint32_t)BM, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUtensorMapDataType dt =
+        dtype == FLASHCK_DTYPE_BFLOAT16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    const CUresult r = enc(map, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    FCK_REQUIRE(r == CUDA_SUCCESS, FLASHCK_ERR_CUDA, "cuTensorMapEncodeTiled (bias) failed (%d) rows=%lld keys=%lld", (int)r,
+                (long long)rows, (long long)keys);
+    return FLASHCK_OK;
+}
+
 template <typename T, int EXPM, int VAR, int SPLIT, int HDIM = 128>
 int launch_t(const FwdParams& p, const Sm100Dev& dev, cudaStream_t stream) {
     const int64_t rows_q = p.seqstart_q ? p.total_q : p.batch * p.seqlen_q;
@@ -1963,7 +2033,14 @@ int launch_t(const FwdParams& p, const Sm100Dev& dev, cudaStream_t stream) {
     }
     if (p.max_seqlen_q == 0 || p.batch == 0) return FLASHCK_OK;
     // persistent: one CTA per SM walks the device-side work list
-    FCK_CUDA(launch_dependent(kern, dim3(sm_count()), dim3(NTHREADS), smem, stream, mq, mk, mv, mo, dev));
+    if constexpr ((VAR & 8) != 0) {
+        Sm100DevBias dev_bias{dev, {}};
+        const int64_t planes = dev.bias_el_rank == 0 ? 1 : dev.bias_el_rank == 1 ? p.hq : p.batch * p.hq;
+        if ((rc = make_map_bias(&dev_bias.map_bias, dev.bias_el, p.dtype, planes, dev.bias_sq, dev.bias_sk))) return rc;
+        FCK_CUDA(launch_dependent(kern, dim3(sm_count()), dim3(NTHREADS), smem, stream, mq, mk, mv, mo, dev_bias));
+    } else {
+        FCK_CUDA(launch_dependent(kern, dim3(sm_count()), dim3(NTHREADS), smem, stream, mq, mk, mv, mo, dev));
+    }
     return FLASHCK_OK;
 }
 
@@ -2019,6 +2096,7 @@ int launch_split_t(const SplitKVParams& p, const Sm100Dev& dev, cudaStream_t str
 #define FCK_SM100_EXTRA(X, T) X(T, 0, 2, 0, 128) X(T, 0, 3, 0, 128)
 #define FCK_SM100_EXTRA64(X, T) X(T, 0, 2, 0, 64) X(T, 0, 3, 0, 64)
 #define FCK_SM100_BIAS(X, T) X(T, 0, 4, 0, 128) X(T, 0, 5, 0, 128)
+#define FCK_SM100_TMA_BIAS(X, T) X(T, 0, 12, 0, 128) X(T, 0, 13, 0, 128)
 #define FCK_SM100_FP8(X, T) X(T, 0, 0, 0, 128) X(T, 0, 1, 0, 128)
 #define FCK_SM100_SPLIT(X, T) X(T, 1, 0) X(T, 1, 1) X(T, 2, 0) X(T, 2, 1)
 #define FCK_SM100_INST(T, E, V, S, H) template int launch_t<T, E, V, S, H>(const FwdParams&, const Sm100Dev&, cudaStream_t);
