@@ -122,6 +122,81 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineDev p) {
     if (p.lse && lane == 0) p.lse[item] = m + logf(sum);
 }
 
+// Two rows per warp, for at most 16 splits and 128 columns (most merges: many rows of a few splits): half a warp holds a row's LSEs,
+// one a lane, so that maximum, sum and weights need no second look at memory, and its 16 lanes take two float4 of every partial
+// row.  The first kFirst splits' rows are requested before the LSEs have come (nearly every row has that many; an empty split's
+// slot may hold anything and is dropped by its weight).  What bounds it is two memory round trips per warp and the waves of
+// warps: behind 270 tokens of 32 heads in 16 slots, 2-6 of them in use, append + split + merge 237 -> 229 us; 48 rows x 32 heads in 8
+// slots at hdim 64, split + merge 74.6 -> 72.6.  The order of the sums is that of combine_kernel.
+template <typename T>
+__global__ void __launch_bounds__(128) combine_pair_kernel(const CombineDev p) {
+    constexpr int kFirst = 2;
+    const int lane = threadIdx.x & 31, sub = lane & 15;
+    const int64_t item = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 2 + (lane >> 4);
+    const bool exists = item < p.items;
+    const int64_t it = exists ? item : p.items - 1;  // (an odd last row: the other half walks along and stores nothing)
+    const int r = (int)(it % p.rows);
+    const int64_t bh = it / p.rows;
+    const int h = (int)(bh % p.hq);
+    const int64_t b = bh / p.hq;
+    const int S = p.S, nvec = p.dv >> 2;
+    const float* lrow = p.lse_acc + b * p.lb + h * p.lh + r * p.lr;
+    const float4* obase = reinterpret_cast<const float4*>(p.o_acc + b * p.ob + h * p.oh + r * p.orr);
+    const int64_t os4 = p.os >> 2;
+    const bool c0 = sub < nvec, c1 = sub + 16 < nvec;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float ninf = -INFINITY;
+    pdl_wait();  // the split kernel's partials are complete and visible (no-op after an ordinary launch)
+
+    float4 x[4][2];
+#pragma unroll
+    for (int u = 0; u < kFirst; ++u) {
+        x[u][0] = (u < S && c0) ? obase[u * os4 + sub] : zero;
+        x[u][1] = (u < S && c1) ? obase[u * os4 + sub + 16] : zero;
+    }
+    const float ls = sub < S ? lrow[sub * p.ls] : ninf;
+    float m = ls;
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    const float e = (ls == ninf) ? 0.f : expf(ls - m);
+    float sum = e;
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    const float wl = m == ninf ? 0.f : e * (1.f / sum);
+    // splits in use by either row of the warp
+    const uint32_t used = __ballot_sync(0xffffffffu, ls != ninf);
+    const int cnt = 32 - __clz((used | used >> 16) & 0xffffu);
+
+    float4 acc[2] = {zero, zero};
+    for (int j0 = 0; j0 < cnt; j0 += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (j0 == 0 && u < kFirst) continue;
+            const bool live = used >> ((lane & 16) + ((j0 + u) & 15)) & 1u;  // (only splits below S are in use)
+            x[u][0] = (live && c0) ? obase[(j0 + u) * os4 + sub] : zero;
+            x[u][1] = (live && c1) ? obase[(j0 + u) * os4 + sub + 16] : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float w = __shfl_sync(0xffffffffu, wl, (lane & 16) + ((j0 + u) & 15));
+            if (w != 0.f) {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    acc[j].x += w * x[u][j].x;
+                    acc[j].y += w * x[u][j].y;
+                    acc[j].z += w * x[u][j].z;
+                    acc[j].w += w * x[u][j].w;
+                }
+            }
+        }
+    }
+    if (!exists) return;
+    T* orow = (T*)p.o + ((b * p.rows + r) * p.hq + h) * (int64_t)p.dv;
+    if (c0) Out4<T>::store(orow + 4 * sub, acc[0]);  // (no split saw a key: zeros)
+    if (c1) Out4<T>::store(orow + 4 * (sub + 16), acc[1]);
+    if (p.lse && sub == 0) p.lse[item] = m == ninf ? ninf : m + logf(sum);
+}
+
 // Several warps per row (one CTA = one row), for rows with many splits: a warp that walks 94 splits four rows at a time
 // pays a memory round trip for every four.  Warp w takes splits w, w + W, ...; it requests its first kAhead rows before
 // it has seen any LSE (a split without keys may hold anything: its row is dropped by its weight of zero, not multiplied),
@@ -191,6 +266,8 @@ __global__ void __launch_bounds__(W * 32) combine_wide_kernel(const CombineDev p
     for (int j0 = 0; j0 * W + warp < S; j0 += kAhead) {
         if (j0 > 0) {
             if ((j0 & 31) == 0) mine = (j0 + lane) * W + warp < S ? lrow[(int64_t)((j0 + lane) * W + warp) * p.ls] : ninf;
+            // (the splits in use come first: behind them there is nothing to fetch)
+            if (!__any_sync(0xffffffffu, mine != ninf && lane >= (j0 & 31) && lane < (j0 & 31) + kAhead)) continue;
             fetch(j0);
         }
         const float wl = (mine == ninf) ? 0.f : expf(mine - m) * inv;
@@ -236,6 +313,9 @@ cudaError_t launch_t(const CombineDev& d, cudaStream_t stream) {
     if (warps_ok >= 8 && d.S > 16) return launch_dependent(combine_wide_kernel<T, 8>, g, dim3(256), 8 * row, stream, d);
     if (warps_ok >= 4 && d.S > 8) return launch_dependent(combine_wide_kernel<T, 4>, g, dim3(128), 4 * row, stream, d);
     const int warps = 4;
+    if (d.S <= 16 && d.dv <= 128)
+        return launch_dependent(combine_pair_kernel<T>, dim3((unsigned)((d.items + 2 * warps - 1) / (2 * warps))),
+                                dim3(warps * 32), 0, stream, d);
     return launch_dependent(combine_kernel<T>, dim3((unsigned)((d.items + warps - 1) / warps)), dim3(warps * 32), 0, stream, d);
 }
 
