@@ -165,6 +165,28 @@ splitkv_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     }
     const int num_pieces = sc.per_batch ? p.batch : (sc.total + sc.piece - 1) / sc.piece;
 
+    // ---- unused splits get LSE = -inf -------------------------------------------------------------
+    if (p.lse_acc && blockIdx.y == 0 && blockIdx.z == 0) {
+        for (int b = blockIdx.x; b < p.batch; b += gridDim.x) {
+            const int n = sm_prefix[b + 1] - sm_prefix[b];
+            int used;
+            if (n == 0) used = 0;
+            else if (sc.per_batch) used = 1;
+            else used = (sm_prefix[b + 1] - 1) / sc.piece - sm_prefix[b] / sc.piece + 1;
+            const int sq = seq_len_q(p, b);
+            const int64_t q0 = p.seqstart_q ? p.seqstart_q[b] : 0;
+            const int cnt = (p.num_splits - used) * sq * p.hq;
+            for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
+                const int i = e % sq;
+                const int s = used + (e / sq) % (p.num_splits - used);
+                const int h = e / (sq * (p.num_splits - used));
+                const int64_t idx = p.seqstart_q ? ((int64_t)h * p.num_splits + s) * p.total_q + q0 + i
+                                                 : (((int64_t)b * p.hq + h) * p.num_splits + s) * p.seqlen_q + i;
+                p.lse_acc[idx] = -INFINITY;
+            }
+        }
+    }
+
     const int hgroup = blockIdx.z;  // kv heads [hgroup*HK, hgroup*HK + HK)
 
     if (warp == HK * MT) {
@@ -239,30 +261,6 @@ splitkv_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                         if (!ok) return;
                         ++it;
                     }
-                }
-            }
-        }
-        // ---- unused splits get LSE = -inf: by the producer warps, which have nothing left to do while the consumers work on the
-        // last tiles (one short conversation leaves thousands of slots: a microsecond where the consumers come to it first) ----
-        if (p.lse_acc && blockIdx.y == 0 && blockIdx.z == 0) {
-            // a sequence's slots are shared out over gridDim.x / batch CTAs
-            const int parts = max(1, (int)gridDim.x / p.batch), part = (int)blockIdx.x / p.batch;
-            for (int b = parts > 1 ? (int)blockIdx.x % p.batch : (int)blockIdx.x; b < p.batch && (parts == 1 || part < parts); b += gridDim.x) {
-                const int n = sm_prefix[b + 1] - sm_prefix[b];
-                int used;
-                if (n == 0) used = 0;
-                else if (sc.per_batch) used = 1;
-                else used = (sm_prefix[b + 1] - 1) / sc.piece - sm_prefix[b] / sc.piece + 1;
-                const int sq = seq_len_q(p, b);
-                const int64_t q0 = p.seqstart_q ? p.seqstart_q[b] : 0;
-                const int cnt = (p.num_splits - used) * sq * p.hq;
-                for (int e = (parts > 1 ? part * 32 : 0) + lane; e < cnt; e += parts * 32) {
-                    const int i = e % sq;
-                    const int s = used + (e / sq) % (p.num_splits - used);
-                    const int h = e / (sq * (p.num_splits - used));
-                    const int64_t idx = p.seqstart_q ? ((int64_t)h * p.num_splits + s) * p.total_q + q0 + i
-                                                     : (((int64_t)b * p.hq + h) * p.num_splits + s) * p.seqlen_q + i;
-                    p.lse_acc[idx] = -INFINITY;
                 }
             }
         }
@@ -595,12 +593,9 @@ int launch_inst(const SplitKVParams& p, const DecodeDev& dev_in, cudaStream_t st
     }
     const int G = (int)(p.hq / p.hkv);
     const int mtiles = (int)((p.max_seqlen_q * G + 16 * MT - 1) / (16 * MT));
-    // one CTA per SM over all groups of heads and row tiles: 16 kv heads, 8 x 2-8k keys 75 -> 72 us, one sequence of 3k 15.6 -> 11.3;
-    // 12 kv heads, 6 x 2-9k 58 -> 50; hdim 64 with 64 rows, 8 x 2-8k 77 -> 61
-    const int groups = (int)(p.hkv / HK);
-    int gx = (int)((int64_t)sm_count() * g_ctas_per_sm_x100.load() / 100) / (groups * mtiles);
+    int gx = (int)((int64_t)sm_count() * g_ctas_per_sm_x100.load() / 100);
     if (gx < 1) gx = 1;
-    dim3 grid(gx, mtiles, (unsigned)groups);
+    dim3 grid(gx, mtiles, (unsigned)(p.hkv / HK));
     FCK_CUDA(launch_dependent(kern, grid, dim3((HK * MT + 1) * 32), smem, stream, mk, mv, dev));
     return FLASHCK_OK;
 }
@@ -615,13 +610,7 @@ int launch_hk(const SplitKVParams& p, const DecodeDev& dev, cudaStream_t stream)
     // the instance parameter caps the heads per CTA; a value the problem cannot take (not a divisor of nhead_k, more
     // than 8 warps with this many row tiles) falls through to the next smaller one
     const int64_t want = g_heads_per_cta.load();
-    // Four heads per CTA where the caches cannot hold much: a CTA's piece is then twice as many tiles of half the heads, which
-    // halves the splits that the merge has to read and the first tile's latency (one sequence of 2-4k keys, split and merge 11.3
-    // against 10.1 us; 2 x 21k 36 / 30; 2 x 32k 52 / 50).  With more keys the 32 KB pieces of a page's eight heads stream better
-    // (3 x 61k 120 / 126; 64 x 1-32k 618 / 662), and at hdim 64 (half the bytes) they always do (48 x 0.3-8k 75 / 84).
-    const int64_t cached = p.batch * (p.block_table ? p.bt_stride * p.page : p.seqlen_k_cap);
-    const bool few = D == 128 && !p.seqstart_k && cached <= 98304;
-    const int cap = want > 0 ? (int)want : few ? 4 : 8;
+    const int cap = want > 0 ? (int)want : 8;
     if constexpr (kMaxHK >= 8) {
         if (cap >= 8 && hkv % 8 == 0) return launch_inst<T, D, 8, MT>(p, dev, stream);
     }
