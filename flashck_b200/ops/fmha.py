@@ -15,6 +15,10 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import glob
+import os
+import sys
+import warnings
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -82,23 +86,43 @@ def _on(device: torch.device):
 
 # Plain calls run in the compiled binding (csrc/pybind/calls.cpp: the same checks, allocations and C call; 2 x 128 tokens 24 us a
 # call in Python, 7.0 there).  It answers None for a call that it cannot check completely; the code below then takes it.
-_NATIVE = None  # the binding, or False where it has not been built
+_NATIVE = None  # the binding, or False where there is none of this package's age that loads
+_NATIVE_CALLS = ("_call_forward", "_call_paged_prefill", "_call_splitkv", "_call_append_kv")
 _TUNING_DIR = flags.flag("FC_TUNING_DB_DIR")  # (set: the call may have to tune first)
 
 
 def _native():
-    """The compiled binding, or False: not built, or tuning is on."""
-    global _NATIVE
+    """The compiled binding, or False: not built, built before the calls it is asked for, not loadable, or tuning is on."""
     if _TUNING_DIR.value:
         return False
-    if _NATIVE is None:
-        _lib.lib()
-        try:
-            from .. import flash_ck
+    return _load_native() if _NATIVE is None else _NATIVE
+
+
+def _load_native():
+    """Looks for the binding once.  A file that is there and cannot be used is worth a warning: every call works without it, but
+    short ones take up to four times as long.  (Not built at all is a choice, ``python -m flashck_b200.build --no-pybind``, and is
+    said under ``FC_TUNING_LOG`` only.)"""
+    global _NATIVE
+    if not os.path.exists(_lib.LIB_PATH):
+        return False  # (not kept: the call itself says so once its arguments have been checked)
+    _NATIVE, why = False, None
+    try:
+        from .. import flash_ck
+        missing = [n for n in _NATIVE_CALLS if not hasattr(flash_ck, n)]
+        if not missing:
+            _lib.lib()
             _NATIVE = flash_ck
-        except ImportError:
-            _NATIVE = False
-    return _NATIVE
+            return _NATIVE
+        why = f"{flash_ck.__name__} has no {', '.join(missing)}: it was built from older sources"
+    except ImportError as e:
+        if glob.glob(os.path.join(os.path.dirname(_lib.LIB_PATH), "flash_ck*.so")):
+            why = f"it cannot be loaded ({e})"
+        elif flags.get_flag("FC_TUNING_LOG"):
+            print("[flashck_b200] the compiled binding has not been built: calls are made from Python", file=sys.stderr)
+    if why:
+        warnings.warn(f"the compiled binding is not used, and short calls are slower: {why}; build it again with "
+                      "`python -m flashck_b200.build`", RuntimeWarning, stacklevel=4)
+    return False
 
 
 def _mask(causal: bool, window_size: Sequence[int], mask_type: Optional[int]) -> Tuple[int, int, int]:
