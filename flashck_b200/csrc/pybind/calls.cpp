@@ -295,16 +295,15 @@ PyObject* call_append_kv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const at::Tensor *v = r.need(elem, 4), *knew = r.need(elem), *vnew = r.need(elem), *sl = r.need(at::kInt);
     const at::Tensor *cos = r.maybe(elem, 2), *sin = r.maybe(elem, 2);
     const int64_t rope = r.integer();
-    int64_t rotary_dim = -1;
-    if (r.i < nargs && args[r.i] == Py_None) ++r.i;
-    else rotary_dim = r.integer();
+    PyObject* width = r.next();  // rotary_dim: None is the tables' width; a number goes to the C call as it is, which refuses a bad one
+    int64_t rotary_dim = width == Py_None ? 0 : r.integer(width);
     const at::Tensor *bt = r.maybe(at::kInt, 2), *cu_q = r.maybe(at::kLong), *cu_n = r.maybe(at::kLong);
     if (!r.ok || r.i != nargs || (q && q->scalar_type() != elem) || (cu_q != nullptr) != (cu_n != nullptr)) Py_RETURN_NONE;
     const int64_t dim = cu_n ? 3 : 4;
     if (knew->dim() != dim || vnew->dim() != dim || (q && q->dim() != dim) || (rope != 0 && (!cos || !sin))) Py_RETURN_NONE;
     const int64_t batch = sl->numel(), hkv = knew->size(-2), d = knew->size(-1), dv = vnew->size(-1);
     const int64_t n_new = cu_n ? knew->size(0) : knew->size(1), sq = !q ? 0 : cu_n ? q->size(0) : q->size(1);
-    if (rotary_dim < 0) rotary_dim = rope != 0 ? 2 * cos->size(1) : 0;
+    if (width == Py_None && rope != 0) rotary_dim = 2 * cos->size(1);
     int rc;
     {
         pybind11::gil_scoped_release no_gil;
