@@ -97,6 +97,9 @@ def build_pybind(force: bool = False) -> str:
         cmd += ["-isystem" if "torch" in inc or "cuda" in inc else "-I", inc]
     cmd += [*srcs, "-o", out, "-L", torch_lib, "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-ltorch_python",
             "-L", HERE, "-l:libflashck_b200.so", f"-Wl,-rpath,{torch_lib}", "-Wl,-rpath,$ORIGIN"]
+    # The C++ library that torch is loaded with, by name: a compiler that finds an archive only links its own copy into the module, and
+    # the two copies' streams then end the process where an error message prints a number.
+    cmd += ["-nostdlib++", "-l:libstdc++.so.6", "-lm"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for {srcs}:\n{r.stdout}\n{r.stderr[-6000:]}")
