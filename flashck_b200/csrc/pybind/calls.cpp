@@ -2,9 +2,9 @@
 //
 // Around a short attention call the Python of ops/fmha.py (checks, torch.empty, argument conversion) takes two to four times as
 // long as its kernels: 2 x 128 tokens 24 us a call with 7 us on the GPU, a decode step of one sequence (two launches) 45 us with
-// 10 us on the GPU.  Here the same calls take 7.0 and 11.6 us.  A function takes only what it can check completely -- exact
-// torch.Tensor objects that are dense, contiguous, on one CUDA device and of the expected shapes and types, Python bools, ints
-// and floats -- and returns None for everything else (subclasses, functorch wrappers, active modes or tracing, other argument
+// 10 us on the GPU.  Here the same calls take 7.0 and 11.6 us.  A function takes only what the host can check completely -- exact
+// torch.Tensor objects that are dense, contiguous, on one CUDA device, of the expected types and of sizes that fit one another (what
+// lies in device memory, lengths and page ids, is the caller's), Python bools, ints and floats -- and returns None for everything else (subclasses, functorch wrappers, active modes or tracing, other argument
 // types, shapes that do not fit); the caller then goes on in Python, which converts, or raises what it always raised.
 // Otherwise it returns the result, or the non-zero status of the C call.
 #include <ATen/ATen.h>
@@ -115,6 +115,11 @@ struct Reader {
     }
 };
 
+bool holds(const at::Tensor* t, int64_t entries) { return !t || t->numel() >= entries; }
+// The same sizes in all dimensions but the last: what a kernel that is given one tensor's sizes takes for the other's too.
+bool same_rows(const at::Tensor& a, const at::Tensor& b) {
+    return a.dim() == b.dim() && a.sizes().slice(0, a.dim() - 1) == b.sizes().slice(0, b.dim() - 1);
+}
 void* ptr(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
 void* ptr(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 int dtype_code(const at::Tensor& t) { return t.scalar_type() == at::kHalf ? FLASHCK_DTYPE_FLOAT16 : FLASHCK_DTYPE_BFLOAT16; }
@@ -206,6 +211,7 @@ PyObject* call_paged_prefill(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     if (q->dim() != (group ? 3 : 4) || (!group && q->size(0) != bt->size(0))) Py_RETURN_NONE;
     const int64_t batch = bt->size(0), hq = q->size(-2), d = q->size(-1), dv = v->size(3);
     const int64_t sq = group ? q->size(0) : q->size(1);
+    if (k->size(3) != d || !same_rows(*k, *v) || !holds(sl, batch) || !holds(cu_q, batch + 1)) Py_RETURN_NONE;
     if (!group || max_q == 0) max_q = sq;
     at::Tensor o, lse;
     int rc;
@@ -251,7 +257,8 @@ PyObject* call_splitkv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (q->dim() != (group ? 3 : 4) || (bt && !sl)) Py_RETURN_NONE;
     const int64_t hq = q->size(-2), d = q->size(-1), hkv = k->size(2), dv = v->size(3);
     const int64_t batch = group ? cu_q->numel() - 1 : q->size(0), sq = group ? q->size(0) : q->size(1);
-    if (batch < 1 || k->size(3) != d || (bt && bt->size(0) != batch)) Py_RETURN_NONE;
+    if (batch < 1 || k->size(3) != d || !same_rows(*k, *v) || !holds(sl, batch)) Py_RETURN_NONE;
+    if (bt ? bt->size(0) != batch : k->size(0) < batch) Py_RETURN_NONE;
     if (!group || max_q == 0) max_q = sq;
     if (splits <= 0) splits = num_splits_for(batch, max_q * (hq / std::max<int64_t>(hkv, 1)));
     const int64_t page = bt ? k->size(1) : 0, bs = group ? 1 : batch;
@@ -303,6 +310,12 @@ PyObject* call_append_kv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (knew->dim() != dim || vnew->dim() != dim || (q && q->dim() != dim) || (rope != 0 && (!cos || !sin))) Py_RETURN_NONE;
     const int64_t batch = sl->numel(), hkv = knew->size(-2), d = knew->size(-1), dv = vnew->size(-1);
     const int64_t n_new = cu_n ? knew->size(0) : knew->size(1), sq = !q ? 0 : cu_n ? q->size(0) : q->size(1);
+    if (!same_rows(*knew, *vnew) || !same_rows(*k, *v) || k->size(2) != hkv || k->size(3) != d || v->size(3) != dv) Py_RETURN_NONE;
+    if (cu_n ? !holds(cu_n, batch + 1) || !holds(cu_q, batch + 1) : knew->size(0) < batch) Py_RETURN_NONE;
+    if ((bt ? bt->size(0) : k->size(0)) < batch) Py_RETURN_NONE;
+    if (rope != 0 && (sin->size(1) != cos->size(1) || (width != Py_None && 2 * cos->size(1) < rotary_dim && rotary_dim <= d) ||
+                      (q && (q->size(-1) != d || (!cu_n && q->size(0) < batch)))))
+        Py_RETURN_NONE;
     if (width == Py_None && rope != 0) rotary_dim = 2 * cos->size(1);
     int rc;
     {

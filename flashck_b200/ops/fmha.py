@@ -155,6 +155,17 @@ def _as_i32(name: str, t: torch.Tensor) -> torch.Tensor:
     return t
 
 
+# The kernels index these by the sizes of other tensors and are told none of their extents.
+def _check_entries(name: str, t: Optional[torch.Tensor], need: int) -> None:
+    if t is not None and t.numel() < need:
+        raise ValueError(f"{name} must have at least {need} entries, got {t.numel()}")
+
+
+def _check_sequences(name: str, t: Optional[torch.Tensor], need: int) -> None:
+    if t is not None and t.shape[0] < need:
+        raise ValueError(f"{name} must have a row for each of the {need} sequences, got shape {tuple(t.shape)}")
+
+
 # --------------------------------------------------------------------------------------------
 # dense / varlen forward
 # --------------------------------------------------------------------------------------------
@@ -298,6 +309,7 @@ def fmha_fwd_fp8(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale_s: 
         batch, (total_q, hq, d), (total_k, hkv, _) = cu_q.numel() - 1, q.shape, k.shape
         sq, sk, max_sq = total_q, total_k, int(max_seqlen_q) or total_q
         o_shape, lse_shape = (total_q, hq), (hq, total_q)
+        _check_entries("cu_seqlens_k", cu_k, batch + 1)
     else:
         if q.dim() != 4:
             raise ValueError("q, k, v must be [batch, seqlen, heads, hdim]")
@@ -305,6 +317,9 @@ def fmha_fwd_fp8(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale_s: 
         batch, sq, hq, d = q.shape
         sk, hkv, max_sq = k.shape[1], k.shape[2], sq
         o_shape, lse_shape = (batch, sq, hq), (batch, hq, sq)
+        _check_sequences("k", k, batch)
+    if k.dim() != q.dim() or k.shape[-1] != d or v.shape[:-1] != k.shape[:-1]:
+        raise ValueError(f"inconsistent shapes q{tuple(q.shape)} k{tuple(k.shape)} v{tuple(v.shape)}")
     dv = v.shape[-1]
     mt, wl, wr = _mask(causal, window_size, mask_type)
     o = torch.empty(o_shape + (dv,), dtype=out_dtype, device=q.device)
@@ -444,6 +459,11 @@ def fmha_fwd_paged_kv_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
         o_shape, lse_shape = (b, sq, hq), (b, hq, sq)
     pages, page, hkv, dk = k_pool.shape
     dv = v_pool.shape[3]
+    if dk != d or v_pool.shape[:3] != k_pool.shape[:3]:
+        raise ValueError(f"inconsistent shapes q{tuple(q.shape)} k{tuple(k_pool.shape)} v{tuple(v_pool.shape)}")
+    _check_entries("seqlen_k", sl, batch)
+    _check_entries("cu_seqlens_q", cu_q, batch + 1)
+    _check_entries("cache_batch_idx", cbi, batch)
     mt, wl, wr = _mask(causal, window_size, mask_type)
     o = torch.empty(o_shape + (dv,), dtype=q.dtype, device=q.device)
     lse = torch.empty(lse_shape, dtype=torch.float32, device=q.device) if return_lse else None
@@ -602,6 +622,10 @@ def fmha_fwd_splitkv(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     hkv, dv = k_cache.shape[-2], v_cache.shape[-1]
     if k_cache.shape[-1] != d:
         raise ValueError("k_cache hdim differs from q")
+    if v_cache.shape[:-1] != k_cache.shape[:-1]:
+        raise ValueError(f"inconsistent shapes k{tuple(k_cache.shape)} v{tuple(v_cache.shape)}")
+    _check_entries("seqlen_k", sl, batch)
+    _check_entries("cache_batch_idx", cbi, batch)
     if bt is not None:
         if sl is None:
             raise ValueError("paged K/V needs seqlen_k")
@@ -614,6 +638,9 @@ def fmha_fwd_splitkv(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     else:
         page, max_pages = 0, 0
         shape_sk = k_cache.shape[0] if cu_k is not None else k_cache.shape[1]
+        _check_entries("cu_seqlens_k", cu_k, batch + 1)
+        if cu_k is None and cbi is None:
+            _check_sequences("k_cache", k_cache, batch)
     S = int(num_splits) if num_splits and num_splits > 0 else \
         default_num_splits(batch, rows_per_kv_head=max_sq * (hq // max(hkv, 1)))
     if workspace is None:
@@ -621,6 +648,12 @@ def fmha_fwd_splitkv(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     else:
         lse_acc, o_acc = workspace
         S = o_acc.shape[2]
+        for n, t in (("o_acc", o_acc), ("lse_acc", lse_acc)):
+            if t is not None and t.dtype != torch.float32:
+                raise TypeError(f"the workspace {n} must have dtype torch.float32, got {t.dtype}")
+        rows = S * hq * (shape_sq if group else batch * shape_sq)
+        _check_entries("the workspace o_acc", o_acc, rows * dv)
+        _check_entries("the workspace lse_acc", lse_acc, rows)
     mt, wl, wr = _mask(causal, window_size, mask_type)
     bias_ptr, bias_enum, bias_rank = _alibi_args(alibi_slopes, batch, hq)
     # pages of a paged pool, or rows of a contiguous cache (packed K/V: unused): where the K/V tensor maps end
@@ -690,6 +723,28 @@ def fmha_fwd_append_kv(q: Optional[torch.Tensor], k_cache: torch.Tensor, v_cache
         n_new = knew.shape[1]
         sq = q.shape[1] if q is not None else 0
     hq = q.shape[-2] if q is not None else hkv
+    if vnew.shape[:-1] != knew.shape[:-1]:
+        raise ValueError(f"inconsistent shapes knew{tuple(knew.shape)} vnew{tuple(vnew.shape)}")
+    for n, t, w in (("k_cache", k_cache, d), ("v_cache", v_cache, dv)):
+        if t.dim() < 3 or t.shape[:2] != k_cache.shape[:2] or t.numel() != t.shape[0] * t.shape[1] * hkv * w:
+            raise ValueError(f"{n} must be [{'pages, page' if bt is not None else 'rows, tokens'}, {hkv}, {w}] like the other cache "
+                             f"and the new tokens, got {tuple(t.shape)}")
+    if group:
+        _check_entries("cu_seqlens_knew", cu_n, batch + 1)
+        _check_entries("cu_seqlens_q", cu_q, batch + 1)
+    else:
+        _check_sequences("knew", knew, batch)
+    _check_entries("cache_batch_idx", cbi, batch)
+    if cbi is None:
+        _check_sequences(*(("k_cache", k_cache) if bt is None else ("block_table", bt)), batch)
+    if rope != RopeEnum.NONE:
+        if q is not None:
+            if q.shape[-1] != d:
+                raise ValueError(f"q and knew must have the same hdim, got {q.shape[-1]} and {d}")
+            if not group:
+                _check_sequences("q", q, batch)
+        if rotary_sin.shape[-1] != rotary_cos.shape[-1] or (rotary_dim is not None and 2 * rotary_cos.shape[-1] < int(rotary_dim) <= d):
+            raise ValueError(f"the rotary tables must hold rotary_dim / 2 columns, got {tuple(rotary_cos.shape)} and {tuple(rotary_sin.shape)}")
     if rotary_dim is None:
         rotary_dim = 2 * rotary_cos.shape[-1] if rope != RopeEnum.NONE else 0
     if bt is not None:
