@@ -243,8 +243,9 @@ splitkv_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
             }
         }
         // ---- unused splits get LSE = -inf: by the producer warps, which have nothing left to do while the consumers work on the
-        // last tiles, a sequence's slots shared out over gridDim.x / batch CTAs (one short conversation leaves thousands, which
-        // delayed a working CTA: one sequence of 300-900 keys, split and merge, 10.7 -> 8.9 us) ----
+        // last tiles, a sequence's heads shared out over gridDim.x / batch CTAs (one short conversation leaves thousands of slots,
+        // which delayed a working CTA: one sequence of 300-900 keys, split and merge, 10.7 -> 8.9 us).  From 75 sequences on a warp
+        // has a sequence's slots to itself; a lane finds its place (split, row) once and goes through the heads from there ----
         if (p.lse_acc && blockIdx.y == 0 && blockIdx.z == 0) {
             const int parts = max(1, (int)gridDim.x / p.batch), part = parts > 1 ? (int)blockIdx.x / p.batch : 0;
             for (int b = parts > 1 ? (int)blockIdx.x % p.batch : (int)blockIdx.x; b < p.batch && part < parts; b += gridDim.x) {
@@ -254,15 +255,12 @@ splitkv_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
                 else if (sc.per_batch) used = 1;
                 else used = (sm_prefix[b + 1] - 1) / sc.piece - sm_prefix[b] / sc.piece + 1;
                 const int sq = seq_len_q(p, b);
-                const int64_t q0 = p.seqstart_q ? p.seqstart_q[b] : 0;
-                const int cnt = (p.num_splits - used) * sq * p.hq;
-                for (int e = part * 32 + lane; e < cnt; e += parts * 32) {
-                    const int i = e % sq;
-                    const int s = used + (e / sq) % (p.num_splits - used);
-                    const int h = e / (sq * (p.num_splits - used));
-                    const int64_t idx = p.seqstart_q ? ((int64_t)h * p.num_splits + s) * p.total_q + q0 + i
-                                                     : (((int64_t)b * p.hq + h) * p.num_splits + s) * p.seqlen_q + i;
-                    p.lse_acc[idx] = -INFINITY;
+                const int64_t rows = p.seqstart_q ? p.total_q : p.seqlen_q, head = p.num_splits * rows;  // LSEs of a split, of a head
+                float* first = p.lse_acc + (p.seqstart_q ? p.seqstart_q[b] : (int64_t)b * p.hq * head) + used * rows;
+                for (int e = lane; e < (p.num_splits - used) * sq; e += 32) {
+                    const int s = e / sq;
+                    float* at = first + s * rows + (e - s * sq);
+                    for (int h = part; h < p.hq; h += parts) at[h * head] = -INFINITY;
                 }
             }
         }
