@@ -413,19 +413,27 @@ __device__ __forceinline__ void add_f16x2_to(float2& acc, uint32_t v) {
         : "r"(v));
 }
 
-// O *= alpha for the rows of a warp (one accumulator row per thread, HD columns from `tO`).  Out of line: it runs once or twice
-// per row, and in place the softmax loop jumps over its instructions in every step.
-template <int HD>
+// O *= alpha for the rows of a warp (one accumulator row per thread, HD columns from `tO`, COLS at a time).
+template <int COLS>
+__device__ __forceinline__ void rescale_columns(uint32_t tO, float alpha) {
+    uint32_t t[COLS];
+    if constexpr (COLS == 32) tmem_ld32(tO, t);
+    else tmem_ld16(tO, t);
+    tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) t[j] = __float_as_uint(__uint_as_float(t[j]) * alpha);
+    if constexpr (COLS == 32) tmem_st32(tO, t);
+    else tmem_st16(tO, t);
+}
+// Out of line: it runs once or twice per row, and in place the softmax loop jumps over its instructions in every step.  COLS: a
+// round trip each on the chain, and as many registers beside the 128 scores of a row.  Prefill forms 16 (with 32, all keys at hdim 64,
+// 2 x 5000 tokens of 32 heads, 539 -> 566 us, at hdim 128 2 x 3000 248 -> 252); the split forms, which wait for the PV of the step
+// before as well, 32 (scores that grow, 2 x 16-32k keys, 16 tokens of 32 heads: 58.7 us, with 16 59.6, in place 59.6; 64k keys, 4
+// tokens of 64 heads: 105.0, 105.2 and 107.7).
+template <int HD, int COLS>
 __device__ __noinline__ void rescale_rows(uint32_t tO, float alpha) {
 #pragma unroll 1
-    for (int c = 0; c < HD; c += 16) {
-        uint32_t t[16];
-        tmem_ld16(tO + c, t);
-        tmem_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) t[j] = __float_as_uint(__uint_as_float(t[j]) * alpha);
-        tmem_st16(tO + c, t);
-    }
+    for (int c = 0; c < HD; c += COLS) rescale_columns<COLS>(tO + c, alpha);
 }
 
 constexpr int kMaxBatch = 256;    // sequences the on-chip schedule can hold (larger batches use the general instance)
@@ -1663,7 +1671,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     l *= alpha;
                     rescale = true;
                     if constexpr (!F8) {
-                        rescale_rows<HD>(tO, alpha);
+                        rescale_rows<HD, SPLIT ? 32 : 16>(tO, alpha);
                         tmem_wait_st();
                     }
                 }

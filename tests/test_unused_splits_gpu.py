@@ -43,5 +43,5 @@ def test_every_slot_is_written(batch, splits, tokens, hq, hkv, d):
     o, lse = ops.fmha_fwd_splitkv_combine(lse_acc, o_acc, torch.float32, varlen=tokens == "packed", return_lse=True)
     one = ops.fmha_fwd_splitkv(*args, num_splits=1, return_lse=True, **kw)
     assert_lse_close(lse, one[1])
-    # (every P is rounded to 8 bits on either side, 2^-9 of it, and the one side's O as well)
+    # (P is rounded to bf16 on either side, and the one side's O as well)
     assert (o - one[0].float()).abs().max() <= 2.0 ** -9 * (2 * c.v.abs().max().float() + o.abs().max())
