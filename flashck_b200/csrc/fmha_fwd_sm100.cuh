@@ -856,6 +856,14 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     static_assert(!BIAS || (SPLIT == 0 && EXPM == 0 && !F8), "the bias instances are prefill forms with fp32 exponentials");
     constexpr int NPOLY8 = EXPM >= 11 ? EXPM - 10 : 0;
     constexpr bool HEXP = EXPM == 1;
+    // Score additions (not the bias tensors) make a step so long that a second copy of it for masked tiles (see the loop over the
+    // steps) does not stay in the instruction cache: they have one, with a jump over the mask.  2 x 5000 tokens, 16 heads, ALiBi behind
+    // a window of 1023: warps per issue that wait for an instruction 1.44 with two copies, 1.10 with one.  O is rescaled in place
+    // but at hdim 64 without a left window: the call's hand-over of the row cost instructions (with a cap 162.8M executed, 152.8M in
+    // place).  us with two copies and the rescale out of line / now: that call 148 / 136, causal with ALiBi and a cap 352 / 321, with a
+    // cap alone 263 / 256; hdim 64, 32 heads over 8, a cap 458 / 432 (in place 483); 16 x 100 tokens of 32 heads 18.5 / 18.7.
+    constexpr bool ONE_STEP = EXTRA && !BIAS;
+    constexpr bool RESCALE_HERE = ONE_STEP && (HDIM == 128 || WINDOW);
     constexpr bool HALVES = FCK_P_HALVES != 0 && SPLIT == 0;  // P reaches the PV in two halves of 64 keys
 
     // ---- shared memory carve-up ----
@@ -1530,8 +1538,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 else off += (p.bias_el_rank == 2 ? (int64_t)it.b * p.hq * plane : 0) + (int64_t)row * p.bias_sk;
                 if (row_ok) bias_row = reinterpret_cast<const unsigned short*>(p.bias_el) + off;
             }
-            auto step = [&](int n, auto mask_tag) -> bool {
-                constexpr bool MASK = decltype(mask_tag)::value;  // some score of the tile is hidden
+            auto step = [&](int n, auto mask) -> bool {  // mask: some score of the tile is hidden (a constant where the step has two copies)
                 // warp-uniform outcome: the loads, votes and stores below are warp-collective
                 // The split modes have one Q tile and use the other tile's S columns as a second S buffer: the QK^T of
                 // step n+1 is issued before the PV of step n, so the next S is there when P has been handed over.
@@ -1629,7 +1636,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 }
                 // Mask: a warp's 32 rows see a prefix (or, with a left window, a band) of the columns, so most 32-column groups
                 // are seen by all of them or by none.
-                if constexpr (MASK) {
+                if (mask) {
                     const int hi = row_ok ? limit - key0 : -1, lo = WINDOW ? first_key - key0 : 0;
 #pragma unroll
                     for (int c = 0; c < NC / 32; ++c) {
@@ -1670,10 +1677,13 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     alpha = grow ? fast_exp2(m_used - mx) : 1.f;  // exp2(-inf) = 0
                     l *= alpha;
                     rescale = true;
-                    if constexpr (!F8) {
+                    if constexpr (RESCALE_HERE) {
+#pragma unroll
+                        for (int c = 0; c < HD; c += 32) rescale_columns<32>(tO + c, alpha);
+                    } else if constexpr (!F8) {
                         rescale_rows<HD, SPLIT ? 32 : 16>(tO, alpha);
-                        tmem_wait_st();
                     }
+                    if constexpr (!F8) tmem_wait_st();
                 }
                 if (grow) m_used = mx;
                 const float msub = (m_used == -INFINITY) ? 0.f : m_used;
@@ -1684,7 +1694,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 // exact zeros for them.
                 auto exp_half = [&](int c, auto rescale_tag) {
                     [[maybe_unused]] constexpr bool RESCALE = decltype(rescale_tag)::value;
-                    [[maybe_unused]] constexpr int NP = MASK ? 0 : NPOLY8;
+                    [[maybe_unused]] constexpr int NP = std::is_same<decltype(mask), std::false_type>::value ? NPOLY8 : 0;
                     if constexpr (F8) {
                         // 8-bit P: stretched by scale_p, rounded (saturating) to the operand format, four keys per
                         // TMEM column; the row sum takes the unrounded values
@@ -1776,10 +1786,10 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                 if (lane == 0) mbar_arrive(HALVES ? &ctrl->p_full2[sb] : &ctrl->p_full[sb]);
                 return true;
             };
-            // The diagonal and tail tiles take a copy of the step of their own, so that the others' code is one straight run:
-            // a jump over the 256 instructions of the mask, or over the rescale of O, costs 100-200 clocks of a step's 3250
-            // (now 2950).  us before / after: 16 x 512-4096 tokens causal 998 / 945; hdim 64, 32 x 1025 tokens 313 / 300;
-            // window with a cap 249 / 240; 2 x 2048 with a bias per head 216 / 204; 8-bit operands 918 / 910.
+            // The diagonal and tail tiles take a copy of the step of their own (but see ONE_STEP), so that the others' code is one
+            // straight run: a jump over the 256 instructions of the mask, or over the rescale of O, costs 100-200 clocks of a step's
+            // 3250 (now 2950).  us before / after: 16 x 512-4096 tokens causal 998 / 945; hdim 64, 32 x 1025 tokens 313 / 300;
+            // 2 x 2048 with a bias per head 216 / 204; 8-bit operands 918 / 910.
             constexpr int NCM = SPLIT == 2 ? 64 : 128;
             if constexpr (F8) {
                 // The steps without a hidden score, n_lo .. n_hi - 1, are worked out ahead: 6 % fewer instructions in the loop (873
@@ -1803,7 +1813,8 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
                     const bool need_mask = (key0 + NCM > sk) ||
                                            (p.causal && wr >= 0 && key0 + NCM - 1 > tile_first_row + shift + wr) ||
                                            (WINDOW && p.causal && wl >= 0 && key0 < tile_first_row + BM - 1 + shift - wl);
-                    ok = need_mask ? step(n, std::true_type{}) : step(n, std::false_type{});
+                    if constexpr (ONE_STEP) ok = step(n, need_mask);
+                    else ok = need_mask ? step(n, std::true_type{}) : step(n, std::false_type{});
                 }
             }
             if (!ok) break;
