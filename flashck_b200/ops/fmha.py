@@ -155,15 +155,15 @@ def _as_i32(name: str, t: torch.Tensor) -> torch.Tensor:
     return t
 
 
-# The kernels index these by the sizes of other tensors and are told none of their extents.
-def _check_entries(name: str, t: Optional[torch.Tensor], need: int) -> None:
-    if t is not None and t.numel() < need:
-        raise ValueError(f"{name} must have at least {need} entries, got {t.numel()}")
+# The kernels index these by the sizes of other tensors and are told none of their extents.  (Each `shape` of a tensor costs a quarter
+# of a microsecond, a slice of one more, so the functions below take it once: the checks then cost what they save.)
+def _refuse(name: str, t: torch.Tensor, need: str) -> None:
+    raise ValueError(f"{name} must have {need}, got shape {tuple(t.shape)}")
 
 
-def _check_sequences(name: str, t: Optional[torch.Tensor], need: int) -> None:
-    if t is not None and t.shape[0] < need:
-        raise ValueError(f"{name} must have a row for each of the {need} sequences, got shape {tuple(t.shape)}")
+def _same_rows(a, b) -> bool:
+    """Two shapes (of three dimensions and up) that agree in all but the last one."""
+    return len(a) == len(b) and a[0] == b[0] and a[1] == b[1] and a[-2] == b[-2] and (len(a) <= 4 or a[:-1] == b[:-1])
 
 
 # --------------------------------------------------------------------------------------------
@@ -268,6 +268,7 @@ def fmha_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: Option
 
 
 _F8_CODES = {torch.float8_e4m3fn: _lib.FLOAT8, torch.float8_e5m2: _lib.BFLOAT8}
+_F8_OUT_CODES = {**_F8_CODES, torch.float16: _lib.FLOAT16, torch.bfloat16: _lib.BFLOAT16}
 _F8_MAX = {torch.float8_e4m3fn: 448.0, torch.float8_e5m2: 57344.0}
 
 
@@ -298,7 +299,7 @@ def fmha_fwd_fp8(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale_s: 
     if code is None:
         raise TypeError(f"fmha_fwd_fp8 takes float8_e4m3fn or float8_e5m2 tensors, got {q.dtype}")
     out_dtype = out_dtype or q.dtype
-    out_code = {**_F8_CODES, torch.float16: _lib.FLOAT16, torch.bfloat16: _lib.BFLOAT16}.get(out_dtype)
+    out_code = _F8_OUT_CODES.get(out_dtype)
     if out_code is None:
         raise TypeError(f"out_dtype must be an 8-bit float type, float16 or bfloat16, got {out_dtype}")
     group = cu_seqlens_q is not None
@@ -306,21 +307,26 @@ def fmha_fwd_fp8(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale_s: 
         if q.dim() != 3 or cu_seqlens_k is None:
             raise ValueError("packed q/k/v [total, heads, hdim] need cu_seqlens_q and cu_seqlens_k")
         cu_q, cu_k = _as_i64("cu_seqlens_q", cu_seqlens_q), _as_i64("cu_seqlens_k", cu_seqlens_k)
-        batch, (total_q, hq, d), (total_k, hkv, _) = cu_q.numel() - 1, q.shape, k.shape
+        batch, (total_q, hq, d), ks = cu_q.numel() - 1, q.shape, k.shape
+        total_k, hkv, _ = ks
         sq, sk, max_sq = total_q, total_k, int(max_seqlen_q) or total_q
         o_shape, lse_shape = (total_q, hq), (hq, total_q)
-        _check_entries("cu_seqlens_k", cu_k, batch + 1)
+        if cu_k.numel() <= batch:
+            _refuse("cu_seqlens_k", cu_k, f"{batch + 1} entries")
     else:
         if q.dim() != 4:
             raise ValueError("q, k, v must be [batch, seqlen, heads, hdim]")
         cu_q = cu_k = None
         batch, sq, hq, d = q.shape
-        sk, hkv, max_sq = k.shape[1], k.shape[2], sq
+        ks = k.shape
+        if len(ks) != 4 or ks[0] < batch:
+            _refuse("k", k, f"4 dimensions and a row for each of the {batch} sequences")
+        sk, hkv, max_sq = ks[1], ks[2], sq
         o_shape, lse_shape = (batch, sq, hq), (batch, hq, sq)
-        _check_sequences("k", k, batch)
-    if k.dim() != q.dim() or k.shape[-1] != d or v.shape[:-1] != k.shape[:-1]:
-        raise ValueError(f"inconsistent shapes q{tuple(q.shape)} k{tuple(k.shape)} v{tuple(v.shape)}")
-    dv = v.shape[-1]
+    vs = v.shape
+    if ks[-1] != d or not _same_rows(ks, vs):
+        raise ValueError(f"inconsistent shapes q{tuple(q.shape)} k{tuple(ks)} v{tuple(vs)}")
+    dv = vs[-1]
     mt, wl, wr = _mask(causal, window_size, mask_type)
     o = torch.empty(o_shape + (dv,), dtype=out_dtype, device=q.device)
     lse = torch.empty(lse_shape, dtype=torch.float32, device=q.device) if return_lse else None
@@ -443,7 +449,8 @@ def fmha_fwd_paged_kv_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
     _check_cuda("v_pool", v_pool, q.dtype)
     bt = _as_i32("block_table", block_table)
     sl = _as_i32("seqlen_k", seqlen_k)
-    batch = bt.shape[0]
+    bts = bt.shape
+    batch = bts[0]
     group = cu_seqlens_q is not None
     cu_q = _as_i64("cu_seqlens_q", cu_seqlens_q) if group else None
     cbi = _as_i64("cache_batch_idx", cache_batch_idx) if cache_batch_idx is not None else None
@@ -457,13 +464,17 @@ def fmha_fwd_paged_kv_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
             raise ValueError("q batch and block_table rows differ")
         shape_sq, max_sq = sq, sq
         o_shape, lse_shape = (b, sq, hq), (b, hq, sq)
-    pages, page, hkv, dk = k_pool.shape
-    dv = v_pool.shape[3]
-    if dk != d or v_pool.shape[:3] != k_pool.shape[:3]:
-        raise ValueError(f"inconsistent shapes q{tuple(q.shape)} k{tuple(k_pool.shape)} v{tuple(v_pool.shape)}")
-    _check_entries("seqlen_k", sl, batch)
-    _check_entries("cu_seqlens_q", cu_q, batch + 1)
-    _check_entries("cache_batch_idx", cbi, batch)
+    ks, vs = k_pool.shape, v_pool.shape
+    pages, page, hkv, dk = ks
+    dv = vs[3]
+    if dk != d or not _same_rows(ks, vs):
+        raise ValueError(f"inconsistent shapes q{tuple(q.shape)} k{tuple(ks)} v{tuple(vs)}")
+    if sl.numel() < batch:
+        _refuse("seqlen_k", sl, f"{batch} entries")
+    if group and cu_q.numel() <= batch:
+        _refuse("cu_seqlens_q", cu_q, f"{batch + 1} entries")
+    if cbi is not None and cbi.numel() < batch:
+        _refuse("cache_batch_idx", cbi, f"{batch} entries")
     mt, wl, wr = _mask(causal, window_size, mask_type)
     o = torch.empty(o_shape + (dv,), dtype=q.dtype, device=q.device)
     lse = torch.empty(lse_shape, dtype=torch.float32, device=q.device) if return_lse else None
@@ -471,7 +482,7 @@ def fmha_fwd_paged_kv_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
     with _on(q.device):
         rc = _lib.lib().FmhaFwdPagedKVPrefillEx(_ptr(q), _ptr(k_pool), _ptr(v_pool), bias_ptr, _ptr(o), _ptr(cu_q),
                                                 _ptr(sl), _ptr(bt), _ptr(cbi), batch, shape_sq, hq, hkv, d, dv, max_sq,
-                                                batch * bt.shape[1], page, float(scale or 0.0), wl, wr, mt, _stream(),
+                                                batch * bts[1], page, float(scale or 0.0), wl, wr, mt, _stream(),
                                                 _ptr(lse), _dtype_code(q), bias_enum, bias_rank, pages)
     _lib.check(rc, "FmhaFwdPagedKVPrefill")
     return (o, lse) if return_lse else o
@@ -619,46 +630,56 @@ def fmha_fwd_splitkv(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
             raise ValueError("q must be [b, sq, hq, d]")
         batch, sq, hq, d = q.shape
         shape_sq, max_sq = sq, sq
-    hkv, dv = k_cache.shape[-2], v_cache.shape[-1]
-    if k_cache.shape[-1] != d:
+    ks, vs = k_cache.shape, v_cache.shape
+    hkv, dv = ks[-2], vs[-1]
+    if ks[-1] != d:
         raise ValueError("k_cache hdim differs from q")
-    if v_cache.shape[:-1] != k_cache.shape[:-1]:
-        raise ValueError(f"inconsistent shapes k{tuple(k_cache.shape)} v{tuple(v_cache.shape)}")
-    _check_entries("seqlen_k", sl, batch)
-    _check_entries("cache_batch_idx", cbi, batch)
+    if not _same_rows(ks, vs):
+        raise ValueError(f"inconsistent shapes k{tuple(ks)} v{tuple(vs)}")
+    if sl is not None and sl.numel() < batch:
+        _refuse("seqlen_k", sl, f"{batch} entries")
+    if cbi is not None and cbi.numel() < batch:
+        _refuse("cache_batch_idx", cbi, f"{batch} entries")
     if bt is not None:
         if sl is None:
             raise ValueError("paged K/V needs seqlen_k")
-        if k_cache.dim() != 4 or bt.shape[0] != batch and cbi is None:
+        bts = bt.shape
+        if len(ks) != 4 or bts[0] != batch and cbi is None:
             raise ValueError("paged pools must be [pages, page, hkv, hdim] and block_table [batch, pages_per_seq]")
-        page = k_cache.shape[1]
+        page = ks[1]
         # the reference passes batch * pages_per_seq and recovers the row stride by dividing (:318)
-        max_pages = batch * bt.shape[1]
-        shape_sk = 0
+        max_pages = batch * bts[1]
+        shape_sk, cap_k = 0, bts[1] * page
     else:
         page, max_pages = 0, 0
-        shape_sk = k_cache.shape[0] if cu_k is not None else k_cache.shape[1]
-        _check_entries("cu_seqlens_k", cu_k, batch + 1)
-        if cu_k is None and cbi is None:
-            _check_sequences("k_cache", k_cache, batch)
-    S = int(num_splits) if num_splits and num_splits > 0 else \
-        default_num_splits(batch, rows_per_kv_head=max_sq * (hq // max(hkv, 1)))
+        if cu_k is not None:
+            shape_sk = ks[0]
+            if cu_k.numel() <= batch:
+                _refuse("cu_seqlens_k", cu_k, f"{batch + 1} entries")
+        else:
+            shape_sk = ks[1]
+            if cbi is None and ks[0] < batch:
+                _refuse("k_cache", k_cache, f"a row for each of the {batch} sequences")
+        cap_k = shape_sk
     if workspace is None:
+        S = int(num_splits) if num_splits and num_splits > 0 else \
+            default_num_splits(batch, rows_per_kv_head=max_sq * (hq // max(hkv, 1)))
         lse_acc, o_acc = splitkv_workspace(q, dv, S, cu_q)
     else:
         lse_acc, o_acc = workspace
         S = o_acc.shape[2]
-        for n, t in (("o_acc", o_acc), ("lse_acc", lse_acc)):
-            if t is not None and t.dtype != torch.float32:
-                raise TypeError(f"the workspace {n} must have dtype torch.float32, got {t.dtype}")
         rows = S * hq * (shape_sq if group else batch * shape_sq)
-        _check_entries("the workspace o_acc", o_acc, rows * dv)
-        _check_entries("the workspace lse_acc", lse_acc, rows)
+        if o_acc.numel() < rows * dv:
+            _refuse("the workspace o_acc", o_acc, f"{rows * dv} entries")
+        if lse_acc is not None and lse_acc.numel() < rows:
+            _refuse("the workspace lse_acc", lse_acc, f"{rows} entries")
+        for t in workspace:
+            if t is not None and t.dtype != torch.float32:
+                raise TypeError(f"the workspaces must have dtype torch.float32, got {t.dtype}")
     mt, wl, wr = _mask(causal, window_size, mask_type)
     bias_ptr, bias_enum, bias_rank = _alibi_args(alibi_slopes, batch, hq)
     # pages of a paged pool, or rows of a contiguous cache (packed K/V: unused): where the K/V tensor maps end
-    pool_extent = 0 if cu_k is not None else k_cache.shape[0]
-    cap_k = bt.shape[1] * page if bt is not None else shape_sk
+    pool_extent = 0 if cu_k is not None else ks[0]
     with _on(q.device):
         rc = _launch_tuned(
             "fmha_fwd_split_kv", dict(dtype=_dtype_name(q), mode="group" if group else "batch", batch=batch, hq=hq, hkv=hkv,
@@ -697,7 +718,7 @@ def fmha_fwd_append_kv(q: Optional[torch.Tensor], k_cache: torch.Tensor, v_cache
         if r is not None:
             _lib.check(r, "FmhaFwdAppendKV")
             return q
-    if rope != RopeEnum.NONE and (rotary_cos is None or rotary_sin is None):
+    if rope and (rotary_cos is None or rotary_sin is None):
         raise ValueError("rotary_cos / rotary_sin are required unless rope == RopeEnum.NONE")
     _check_cuda("k_cache", k_cache)
     dt = k_cache.dtype
@@ -709,48 +730,56 @@ def fmha_fwd_append_kv(q: Optional[torch.Tensor], k_cache: torch.Tensor, v_cache
     cbi = _as_i64("cache_batch_idx", cache_batch_idx) if cache_batch_idx is not None else None
     group = cu_seqlens_knew is not None
     batch = sl.numel()
-    hkv, d = knew.shape[-2], knew.shape[-1]
-    dv = vnew.shape[-1]
+    ns, vs, kc, vc = knew.shape, vnew.shape, k_cache.shape, v_cache.shape
+    hkv, d, dv = ns[-2], ns[-1], vs[-1]
+    qs = q.shape if q is not None else None
+    if not _same_rows(ns, vs):
+        raise ValueError(f"inconsistent shapes knew{tuple(ns)} vnew{tuple(vs)}")
     if group:
         cu_n = _as_i64("cu_seqlens_knew", cu_seqlens_knew)
         if cu_seqlens_q is None:
             raise ValueError("varlen append needs cu_seqlens_q together with cu_seqlens_knew")
         cu_q = _as_i64("cu_seqlens_q", cu_seqlens_q)
-        n_new = knew.shape[0]
-        sq = q.shape[0] if q is not None else 0
+        for n, t in (("cu_seqlens_knew", cu_n), ("cu_seqlens_q", cu_q)):
+            if t.numel() <= batch:
+                _refuse(n, t, f"{batch + 1} entries")
+        n_new = ns[0]
+        sq = qs[0] if qs is not None else 0
     else:
         cu_n = cu_q = None
-        n_new = knew.shape[1]
-        sq = q.shape[1] if q is not None else 0
-    hq = q.shape[-2] if q is not None else hkv
-    if vnew.shape[:-1] != knew.shape[:-1]:
-        raise ValueError(f"inconsistent shapes knew{tuple(knew.shape)} vnew{tuple(vnew.shape)}")
-    for n, t, w in (("k_cache", k_cache, d), ("v_cache", v_cache, dv)):
-        if t.dim() < 3 or t.shape[:2] != k_cache.shape[:2] or t.numel() != t.shape[0] * t.shape[1] * hkv * w:
-            raise ValueError(f"{n} must be [{'pages, page' if bt is not None else 'rows, tokens'}, {hkv}, {w}] like the other cache "
-                             f"and the new tokens, got {tuple(t.shape)}")
-    if group:
-        _check_entries("cu_seqlens_knew", cu_n, batch + 1)
-        _check_entries("cu_seqlens_q", cu_q, batch + 1)
-    else:
-        _check_sequences("knew", knew, batch)
-    _check_entries("cache_batch_idx", cbi, batch)
-    if cbi is None:
-        _check_sequences(*(("k_cache", k_cache) if bt is None else ("block_table", bt)), batch)
-    if rope != RopeEnum.NONE:
-        if q is not None:
-            if q.shape[-1] != d:
-                raise ValueError(f"q and knew must have the same hdim, got {q.shape[-1]} and {d}")
-            if not group:
-                _check_sequences("q", q, batch)
-        if rotary_sin.shape[-1] != rotary_cos.shape[-1] or (rotary_dim is not None and 2 * rotary_cos.shape[-1] < int(rotary_dim) <= d):
-            raise ValueError(f"the rotary tables must hold rotary_dim / 2 columns, got {tuple(rotary_cos.shape)} and {tuple(rotary_sin.shape)}")
-    if rotary_dim is None:
-        rotary_dim = 2 * rotary_cos.shape[-1] if rope != RopeEnum.NONE else 0
+        if ns[0] < batch:
+            _refuse("knew", knew, f"a row for each of the {batch} sequences")
+        n_new = ns[1]
+        sq = qs[1] if qs is not None else 0
+    hq = qs[-2] if qs is not None else hkv
+    # the rows of the caches: heads and columns of the new tokens
+    if not (len(kc) == 4 and len(vc) == 4 and kc[2] == hkv and kc[3] == d and vc[2] == hkv and vc[3] == dv):
+        for n, t, c, w in (("k_cache", k_cache, kc, d), ("v_cache", v_cache, vc, dv)):
+            if len(c) < 3 or t.numel() != c[0] * c[1] * hkv * w:
+                _refuse(n, t, f"{hkv} heads of {w} columns, like the new tokens")
+    if kc[0] != vc[0] or kc[1] != vc[1]:
+        raise ValueError(f"inconsistent shapes k_cache{tuple(kc)} v_cache{tuple(vc)}")
     if bt is not None:
-        page, max_pages, cap = k_cache.shape[1], batch * bt.shape[1], 0
+        bts = bt.shape
+        if cbi is None and bts[0] < batch:
+            _refuse("block_table", bt, f"a row for each of the {batch} sequences")
+        page, max_pages, cap = kc[1], batch * bts[1], 0
     else:
-        page, max_pages, cap = 0, 0, k_cache.shape[1]
+        if cbi is None and kc[0] < batch:
+            _refuse("k_cache", k_cache, f"a row for each of the {batch} sequences")
+        page, max_pages, cap = 0, 0, kc[1]
+    if cbi is not None and cbi.numel() < batch:
+        _refuse("cache_batch_idx", cbi, f"{batch} entries")
+    if rope:
+        width = rotary_cos.shape[-1]
+        if qs is not None and (qs[-1] != d or (not group and qs[0] < batch)):
+            _refuse("q", q, f"{d} columns, like knew, and a row for each of the {batch} sequences")
+        if rotary_sin.shape[-1] != width or (rotary_dim is not None and 2 * width < int(rotary_dim) <= d):
+            raise ValueError(f"the rotary tables must hold rotary_dim / 2 columns, got {tuple(rotary_cos.shape)} and {tuple(rotary_sin.shape)}")
+        if rotary_dim is None:
+            rotary_dim = 2 * width
+    elif rotary_dim is None:
+        rotary_dim = 0
     with _on(k_cache.device):
         rc = _lib.lib().FmhaFwdAppendKV(_ptr(q), _ptr(k_cache), _ptr(knew), _ptr(v_cache), _ptr(vnew), _ptr(sl),
                                         _ptr(cu_q), _ptr(cu_n), _ptr(rotary_cos), _ptr(rotary_sin), _ptr(bt),
