@@ -32,6 +32,7 @@ std::atomic<int64_t> g_rescale_half_x100{200};
 
 std::atomic<int64_t> g_use_sm100{1};
 std::atomic<int64_t> g_use_sm100_bias{1};    // elementwise bias tensors (hdim 128, contiguous) on the tcgen05 instance (0: general)
+std::atomic<int64_t> g_last_bias_form{-1};   // how the last bias tensor of this process came: 1 by TMA, 0 by the threads ("last_bias_form", read-only)
 std::atomic<int64_t> g_use_sm100_fp8{1};     // 8-bit prefill (hdim 128, contiguous) on the tcgen05 instance (0: general)
 std::atomic<int64_t> g_use_sm100_hdim64{1};  // hdim-64 prefill on the tcgen05 instance (0: on the general one)
 // exponentials of the softmax (template parameter EXPM of the kernel): 0 fp32 on the exp2 unit, 1 packed f16x2 on the
@@ -172,6 +173,7 @@ int launch_fwd_sm100(const FwdParams& p, cudaStream_t stream) {
         dev.rescale_thr = kRescaleThreshold;
         dev.bias_el = p.bias; dev.bias_el_rank = p.bias_rank;
         dev.bias_sk = p.seqlen_k; dev.bias_sq = p.seqstart_q ? p.total_q : p.seqlen_q;
+        g_last_bias_form = bias_by_tma(p) ? 1 : 0;
         if (bias_by_tma(p)) {
             if (window) return bf16 ? launch_t<__nv_bfloat16, 0, 13, 0>(p, dev, stream) : launch_t<__half, 0, 13, 0>(p, dev, stream);
             return bf16 ? launch_t<__nv_bfloat16, 0, 12, 0>(p, dev, stream) : launch_t<__half, 0, 12, 0>(p, dev, stream);
@@ -322,6 +324,7 @@ int fwd_get_param(const char* key, int64_t* value) {
     if (!strcmp(key, "use_sm100_hdim64")) { *value = g_use_sm100_hdim64; return FLASHCK_OK; }
     if (!strcmp(key, "use_sm100_fp8")) { *value = g_use_sm100_fp8; return FLASHCK_OK; }
     if (!strcmp(key, "use_sm100_bias")) { *value = g_use_sm100_bias; return FLASHCK_OK; }
+    if (!strcmp(key, "last_bias_form")) { *value = g_last_bias_form; return FLASHCK_OK; }
     if (!strcmp(key, "use_sm100_splitkv")) { *value = g_use_sm100_splitkv; return FLASHCK_OK; }
     if (!strcmp(key, "exp_mode")) { *value = g_exp_mode; return FLASHCK_OK; }
     if (!strcmp(key, "exp_mode_splitkv")) { *value = g_exp_mode_splitkv; return FLASHCK_OK; }
