@@ -4,8 +4,9 @@
 // [bs,hq,S,rows], o_acc [bs,hq,S,rows,dv].  The strided form also reads partials gathered from several GPUs
 // ([rank][...] layouts) and can leave the result in fp32, which is what a rank contributes to such a gather.
 // The partials in use are read once: from half a megabyte (one token of 32 heads, 32 splits) to some 10-30 MB (9888 rows of
-// dv 128 with 2-6 splits), mostly out of L2.  What bounds the kernel is its chain of memory round trips: one warp per (batch,
-// head, row) when a row has few splits, several warps per row otherwise (see combine_wide_kernel).
+// dv 128 with 2-6 splits), mostly out of L2.  What bounds the kernel is its chain of memory round trips.  Three forms (launch_t picks):
+// two (batch, head, row) rows per warp for at most 16 splits and 128 columns (combine_pair_kernel), several warps per row for rows
+// with many splits as long as all rows together stay within 16 warps per SM (combine_wide_kernel), one warp per row for the rest.
 #include "kernels.h"
 
 namespace fck {
@@ -201,7 +202,8 @@ __global__ void __launch_bounds__(128) combine_pair_kernel(const CombineDev p) {
 // pays a memory round trip for every four.  Warp w takes splits w, w + W, ...; it requests its first kAhead rows before
 // it has seen any LSE (a split without keys may hold anything: its row is dropped by its weight of zero, not multiplied),
 // so that a row of up to W * kAhead splits costs one round trip for LSE and partials together, and a longer one another for
-// every further W * kAhead.  All slots of a row are read, those of empty splits too.
+// every further W * kAhead.  The LSEs of all slots and the partials of the first W * kAhead are read whether a split has keys or
+// not; of the later ones a warp skips every kAhead in which none has.
 // Merging one token of 32 heads over 128 split slots, 94 in use: 16.4 us with one warp per row, 3.3 us with 16 (back to
 // back in a graph; 24.5 us alone behind its split kernel before).
 template <typename T, int W>

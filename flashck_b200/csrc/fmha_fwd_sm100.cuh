@@ -300,8 +300,8 @@ template <typename T> struct ElemInfo { static constexpr int bytes = 2; static c
 template <> struct ElemInfo<f8e4m3_t> { static constexpr int bytes = 1; static constexpr bool f8 = true; };
 template <> struct ElemInfo<f8e5m2_t> { static constexpr int bytes = 1; static constexpr bool f8 = true; };
 
-// Four values in order, rounded (nearest even, saturating) to the 8-bit format.  (One statement for both conversions: the second
-// one then writes the upper half itself, 828 against 835 us on 16 x 512-4096 tokens.)
+// Four values in order, rounded (nearest even, saturating) to the 8-bit format.  (One statement for both conversions: 828 against 835
+// us on 16 x 512-4096 tokens.)
 template <typename T>
 __device__ __forceinline__ uint32_t pack_f8x4(float2 a, float2 b) {
     uint32_t r;
