@@ -80,7 +80,7 @@ def build_pybind(force: bool = False) -> str:
     srcs = [os.path.join(CSRC, "pybind", f) for f in ("flash_ck.cpp", "calls.cpp")]
     out = os.path.join(HERE, "flash_ck" + sysconfig.get_config_var("EXT_SUFFIX"))
     lib = build()
-    deps = [*srcs, lib, os.path.join(HERE, "..", "include", "flashck", "fmha", "fmha_fwd.h"),
+    deps = [*srcs, lib, os.path.abspath(__file__), os.path.join(HERE, "..", "include", "flashck", "fmha", "fmha_fwd.h"),
             os.path.join(HERE, "..", "include", "flashck_b200.h")]
     if not force and os.path.exists(out) and os.path.getmtime(out) >= _newest(deps):
         return out
