@@ -116,9 +116,9 @@ struct Reader {
 };
 
 bool holds(const at::Tensor* t, int64_t entries) { return !t || t->numel() >= entries; }
-// The same sizes in all dimensions but the last: what a kernel that is given one tensor's sizes takes for the other's too.
-bool same_rows(const at::Tensor& a, const at::Tensor& b) {
-    return a.dim() == b.dim() && a.sizes().slice(0, a.dim() - 1) == b.sizes().slice(0, b.dim() - 1);
+// K and its V: the same sizes in all dimensions but the last, and V may go on behind K's first one.  (The kernels are given K's.)
+bool rows_fit(const at::Tensor& k, const at::Tensor& v) {
+    return k.dim() == v.dim() && k.size(0) <= v.size(0) && k.sizes().slice(1, k.dim() - 2) == v.sizes().slice(1, v.dim() - 2);
 }
 void* ptr(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
 void* ptr(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
@@ -211,7 +211,7 @@ PyObject* call_paged_prefill(PyObject*, PyObject* const* args, Py_ssize_t nargs)
     if (q->dim() != (group ? 3 : 4) || (!group && q->size(0) != bt->size(0))) Py_RETURN_NONE;
     const int64_t batch = bt->size(0), hq = q->size(-2), d = q->size(-1), dv = v->size(3);
     const int64_t sq = group ? q->size(0) : q->size(1);
-    if (k->size(3) != d || !same_rows(*k, *v) || !holds(sl, batch) || !holds(cu_q, batch + 1)) Py_RETURN_NONE;
+    if (k->size(3) != d || !rows_fit(*k, *v) || !holds(sl, batch) || !holds(cu_q, batch + 1)) Py_RETURN_NONE;
     if (!group || max_q == 0) max_q = sq;
     at::Tensor o, lse;
     int rc;
@@ -257,7 +257,7 @@ PyObject* call_splitkv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (q->dim() != (group ? 3 : 4) || (bt && !sl)) Py_RETURN_NONE;
     const int64_t hq = q->size(-2), d = q->size(-1), hkv = k->size(2), dv = v->size(3);
     const int64_t batch = group ? cu_q->numel() - 1 : q->size(0), sq = group ? q->size(0) : q->size(1);
-    if (batch < 1 || k->size(3) != d || !same_rows(*k, *v) || !holds(sl, batch)) Py_RETURN_NONE;
+    if (batch < 1 || k->size(3) != d || !rows_fit(*k, *v) || !holds(sl, batch)) Py_RETURN_NONE;
     if (bt ? bt->size(0) != batch : k->size(0) < batch) Py_RETURN_NONE;
     if (!group || max_q == 0) max_q = sq;
     if (splits <= 0) splits = num_splits_for(batch, max_q * (hq / std::max<int64_t>(hkv, 1)));
@@ -310,7 +310,7 @@ PyObject* call_append_kv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (knew->dim() != dim || vnew->dim() != dim || (q && q->dim() != dim) || (rope != 0 && (!cos || !sin))) Py_RETURN_NONE;
     const int64_t batch = sl->numel(), hkv = knew->size(-2), d = knew->size(-1), dv = vnew->size(-1);
     const int64_t n_new = cu_n ? knew->size(0) : knew->size(1), sq = !q ? 0 : cu_n ? q->size(0) : q->size(1);
-    if (!same_rows(*knew, *vnew) || !same_rows(*k, *v) || k->size(2) != hkv || k->size(3) != d || v->size(3) != dv) Py_RETURN_NONE;
+    if (!rows_fit(*knew, *vnew) || !rows_fit(*k, *v) || k->size(2) != hkv || k->size(3) != d || v->size(3) != dv) Py_RETURN_NONE;
     if (cu_n ? !holds(cu_n, batch + 1) || !holds(cu_q, batch + 1) : knew->size(0) < batch) Py_RETURN_NONE;
     if ((bt ? bt->size(0) : k->size(0)) < batch) Py_RETURN_NONE;
     if (rope != 0 && (sin->size(1) != cos->size(1) || (width != Py_None && 2 * cos->size(1) < rotary_dim && rotary_dim <= d) ||

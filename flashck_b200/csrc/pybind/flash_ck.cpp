@@ -199,7 +199,7 @@ std::tuple<at::Tensor, at::Tensor> fmha_fwd_paged_kv_prefill(at::Tensor q, at::T
         o_shape = {batch, shape_sq, hq, dv}; lse_shape = {batch, hq, shape_sq};
     }
     TORCH_CHECK(seqlen_k.numel() == batch && k_pool.size(3) == d, "seqlen_k must have batch entries; k_pool hdim must match q");
-    TORCH_CHECK(v_pool.size(0) == k_pool.size(0) && v_pool.size(1) == k_pool.size(1) && v_pool.size(2) == k_pool.size(2),
+    TORCH_CHECK(v_pool.size(0) >= k_pool.size(0) && v_pool.size(1) == k_pool.size(1) && v_pool.size(2) == k_pool.size(2),
                 "inconsistent pool shapes k", k_pool.sizes(), " v", v_pool.sizes());
     auto [mask, wl, wr] = resolve_mask(causal, window_left, window_right, mask_type);
     c10::cuda::CUDAGuard guard(q.device());
@@ -222,7 +222,7 @@ std::tuple<at::Tensor, at::Tensor> fmha_fwd_splitkv(at::Tensor q, at::Tensor k_c
     const int64_t b = q.size(0), sq = q.size(1), hq = q.size(2), d = q.size(3);
     const int64_t hkv = k_cache.size(2), dv = v_cache.size(3);
     TORCH_CHECK(k_cache.size(3) == d, "k_cache hdim differs from q");
-    TORCH_CHECK(v_cache.size(0) == k_cache.size(0) && v_cache.size(1) == k_cache.size(1) && v_cache.size(2) == hkv,
+    TORCH_CHECK(v_cache.size(0) >= k_cache.size(0) && v_cache.size(1) == k_cache.size(1) && v_cache.size(2) == hkv,
                 "inconsistent cache shapes k", k_cache.sizes(), " v", v_cache.sizes());
     TORCH_CHECK(!seqlen_k.has_value() || seqlen_k->numel() >= b, "seqlen_k must have batch entries");
     const bool paged = block_table.has_value();
@@ -267,7 +267,7 @@ at::Tensor fmha_fwd_appendkv(at::Tensor q, at::Tensor k_cache, at::Tensor v_cach
     TORCH_CHECK(seqlen_k.numel() == b && knew.size(0) == b && vnew.size(0) == b && vnew.size(1) == n, "inconsistent batch / new-token counts");
     TORCH_CHECK(knew.size(3) == d && vnew.size(2) == hkv, "inconsistent shapes q", q.sizes(), " knew", knew.sizes(), " vnew", vnew.sizes());
     TORCH_CHECK(v_cache.dim() == 4 && k_cache.size(2) == hkv && k_cache.size(3) == d && v_cache.size(2) == hkv && v_cache.size(3) == dv &&
-                    v_cache.size(0) == k_cache.size(0) && v_cache.size(1) == k_cache.size(1),
+                    v_cache.size(0) >= k_cache.size(0) && v_cache.size(1) == k_cache.size(1),
                 "the caches do not fit each other and the new tokens: k_cache", k_cache.sizes(), " v_cache", v_cache.sizes());
     int64_t rotary_dim = 0;
     if (rope != 0) {

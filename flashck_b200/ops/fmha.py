@@ -161,9 +161,9 @@ def _refuse(name: str, t: torch.Tensor, need: str) -> None:
     raise ValueError(f"{name} must have {need}, got shape {tuple(t.shape)}")
 
 
-def _same_rows(a, b) -> bool:
-    """Two shapes (of three dimensions and up) that agree in all but the last one."""
-    return len(a) == len(b) and a[0] == b[0] and a[1] == b[1] and a[-2] == b[-2] and (len(a) <= 4 or a[:-1] == b[:-1])
+def _rows_fit(a, b) -> bool:
+    """The shapes of a K tensor and its V (three dimensions and up) agree in all but the last one; V may go on behind K's first."""
+    return len(a) == len(b) and a[0] <= b[0] and a[1] == b[1] and a[-2] == b[-2] and (len(a) <= 4 or a[1:-1] == b[1:-1])
 
 
 # --------------------------------------------------------------------------------------------
@@ -324,7 +324,7 @@ def fmha_fwd_fp8(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale_s: 
         sk, hkv, max_sq = ks[1], ks[2], sq
         o_shape, lse_shape = (batch, sq, hq), (batch, hq, sq)
     vs = v.shape
-    if ks[-1] != d or not _same_rows(ks, vs):
+    if ks[-1] != d or not _rows_fit(ks, vs):
         raise ValueError(f"inconsistent shapes q{tuple(q.shape)} k{tuple(ks)} v{tuple(vs)}")
     dv = vs[-1]
     mt, wl, wr = _mask(causal, window_size, mask_type)
@@ -467,7 +467,7 @@ def fmha_fwd_paged_kv_prefill(q: torch.Tensor, k_pool: torch.Tensor, v_pool: tor
     ks, vs = k_pool.shape, v_pool.shape
     pages, page, hkv, dk = ks
     dv = vs[3]
-    if dk != d or not _same_rows(ks, vs):
+    if dk != d or not _rows_fit(ks, vs):
         raise ValueError(f"inconsistent shapes q{tuple(q.shape)} k{tuple(ks)} v{tuple(vs)}")
     if sl.numel() < batch:
         _refuse("seqlen_k", sl, f"{batch} entries")
@@ -634,7 +634,7 @@ def fmha_fwd_splitkv(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     hkv, dv = ks[-2], vs[-1]
     if ks[-1] != d:
         raise ValueError("k_cache hdim differs from q")
-    if not _same_rows(ks, vs):
+    if not _rows_fit(ks, vs):
         raise ValueError(f"inconsistent shapes k{tuple(ks)} v{tuple(vs)}")
     if sl is not None and sl.numel() < batch:
         _refuse("seqlen_k", sl, f"{batch} entries")
@@ -733,7 +733,7 @@ def fmha_fwd_append_kv(q: Optional[torch.Tensor], k_cache: torch.Tensor, v_cache
     ns, vs, kc, vc = knew.shape, vnew.shape, k_cache.shape, v_cache.shape
     hkv, d, dv = ns[-2], ns[-1], vs[-1]
     qs = q.shape if q is not None else None
-    if not _same_rows(ns, vs):
+    if not _rows_fit(ns, vs):
         raise ValueError(f"inconsistent shapes knew{tuple(ns)} vnew{tuple(vs)}")
     if group:
         cu_n = _as_i64("cu_seqlens_knew", cu_seqlens_knew)
@@ -757,7 +757,7 @@ def fmha_fwd_append_kv(q: Optional[torch.Tensor], k_cache: torch.Tensor, v_cache
         for n, t, c, w in (("k_cache", k_cache, kc, d), ("v_cache", v_cache, vc, dv)):
             if len(c) < 3 or t.numel() != c[0] * c[1] * hkv * w:
                 _refuse(n, t, f"{hkv} heads of {w} columns, like the new tokens")
-    if kc[0] != vc[0] or kc[1] != vc[1]:
+    if kc[0] > vc[0] or kc[1] != vc[1]:
         raise ValueError(f"inconsistent shapes k_cache{tuple(kc)} v_cache{tuple(vc)}")
     if bt is not None:
         bts = bt.shape

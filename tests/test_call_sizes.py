@@ -110,6 +110,9 @@ FITS = [("append", f, {}) for f in ("paged", "packed", "contiguous")] + [("prefi
     ("append", "paged", {"q": (1, 3, 4, 32), "rope": 0}), ("append", "paged", {"k_cache": (9, 16, 128), "v_cache": (9, 16, 256)}),
     ("append", "contiguous", {"k_cache": (7, 50, 2, 64), "v_cache": (7, 50, 2, 128), "cache_batch_idx": (2,)}),
     ("append", "paged", {"rotary_cos": (40, 16), "rotary_sin": (40, 16)}), ("append", "contiguous", {"k_cache": (3, 50, 2, 64), "v_cache": (3, 50, 2, 128)}),
+    ("append", "paged", {"v_cache": (10, 16, 2, 128)}), ("append", "packed", {"vnew": (7, 2, 128)}), ("prefill", "paged", {"v_pool": (10, 16, 2, 64)}),
+    ("decode", "paged", {"v_cache": (10, 16, 2, 64)}), ("decode", "contiguous", {"v_cache": (3, 50, 2, 64)}),
+    ("decode", "packed keys", {"v_cache": (71, 2, 64)}), ("fp8", "packed", {"v": (71, 2, 64)}),
     ("prefill", "paged", {"seqlen_k": (5,)}), ("prefill", "packed", {"cu_seqlens_q": (6,)}),
     ("decode", "paged", {"seqlen_k": (5,)}), ("decode", "contiguous", {"k_cache": (3, 50, 2, 64), "v_cache": (3, 50, 2, 64)}),
     ("decode", "contiguous", {"k_cache": (1, 50, 2, 64), "v_cache": (1, 50, 2, 64), "cache_batch_idx": (2,)}),
