@@ -429,7 +429,7 @@ __device__ __forceinline__ void rescale_columns(uint32_t tO, float alpha) {
 // round trip each on the chain, and as many registers beside the 128 scores of a row.  Prefill forms 16 (with 32, all keys at hdim 64,
 // 2 x 5000 tokens of 32 heads, 539 -> 566 us, at hdim 128 2 x 3000 248 -> 252); the split forms, which wait for the PV of the step
 // before as well, 32 (scores that grow, 2 x 16-32k keys, 16 tokens of 32 heads: 58.7 us, with 16 59.6, in place 59.6; 64k keys, 4
-// tokens of 64 heads: 105.0, 105.2 and 107.7).
+// tokens of 64 heads: 105.0, 105.2 and 107.7), and so the score additions behind a window at hdim 128 (see RESCALE_HERE).
 template <int HD, int COLS>
 __device__ __noinline__ void rescale_rows(uint32_t tO, float alpha) {
 #pragma unroll 1
@@ -858,12 +858,15 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     constexpr bool HEXP = EXPM == 1;
     // Score additions (not the bias tensors) make a step so long that a second copy of it for masked tiles (see the loop over the
     // steps) does not stay in the instruction cache: they have one, with a jump over the mask.  2 x 5000 tokens, 16 heads, ALiBi behind
-    // a window of 1023: warps per issue that wait for an instruction 1.44 with two copies, 1.10 with one.  O is rescaled in place
-    // but at hdim 64 without a left window: the call's hand-over of the row cost instructions (with a cap 162.8M executed, 152.8M in
-    // place).  us with two copies and the rescale out of line / now: that call 148 / 136, causal with ALiBi and a cap 352 / 321, with a
-    // cap alone 263 / 256; hdim 64, 32 heads over 8, a cap 458 / 432 (in place 483); 16 x 100 tokens of 32 heads 18.5 / 18.7.
+    // a window of 1023: warps per issue that wait for an instruction 1.44 with two copies, 1.10 with one.  Where O is rescaled is the
+    // form that measured best (each 1-5 % ahead of the others): in place at hdim 128 without a left window and at hdim 64 with one, else by
+    // the call, 32 columns at a time behind a window.  us with two copies and the call of 16 columns / now: 2 x 5000 tokens, 16 heads,
+    // causal with ALiBi and a cap 352 / 321 (by the call 336), with a cap 263 / 256; ALiBi behind a window 146 / 133, a cap behind a window,
+    // 32 heads over 8, 222 / 216 (in place 222); hdim 64, 32 heads over 8, a cap 458 / 432 (in place 483); 16 x 100 tokens of 32 heads
+    // 18.5 / 18.7.
     constexpr bool ONE_STEP = EXTRA && !BIAS;
-    constexpr bool RESCALE_HERE = ONE_STEP && (HDIM == 128 || WINDOW);
+    constexpr bool RESCALE_HERE = ONE_STEP && (HDIM == 128) != WINDOW;
+    constexpr int RESCALE_COLS = SPLIT || (ONE_STEP && WINDOW) ? 32 : 16;  // (by the call; see rescale_rows)
     constexpr bool HALVES = FCK_P_HALVES != 0 && SPLIT == 0;  // P reaches the PV in two halves of 64 keys
 
     // ---- shared memory carve-up ----
@@ -1681,7 +1684,7 @@ fmha_fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 #pragma unroll
                         for (int c = 0; c < HD; c += 32) rescale_columns<32>(tO + c, alpha);
                     } else if constexpr (!F8) {
-                        rescale_rows<HD, SPLIT ? 32 : 16>(tO, alpha);
+                        rescale_rows<HD, RESCALE_COLS>(tO, alpha);
                     }
                     if constexpr (!F8) tmem_wait_st();
                 }
